@@ -334,16 +334,16 @@ __global__ void __launch_bounds__(256)
 }
 
 // Ordering of the window's big groups; when hot keys produced groups of
-// more than kSortSmall members, the grid (a cooperative launch) continues
+// more than kHugeSteps members, the grid (a cooperative launch) continues
 // with the huge_* steps between grid barriers.
 // fused_epoch: the window's epoch is the device one (the two-stream form).
 template <class Tr>
 __global__ void __launch_bounds__(1024, 1)
     k_sort(Scratch sc, Window<Tr> w, GridBarrier* bar, const uint32_t* fused_epoch) {
-  extern __shared__ uint32_t smem[];
+  extern __shared__ __align__(16) uint32_t smem[];
   if (fused_epoch != nullptr) w.epoch = 2 * dev_window_slot(fused_epoch) + 1;
   phase_sort_big<Tr>(sc, w, smem);
-  if (huge_groups(sc, w.cnt) == 0) return;  // grid-uniform: the probe kernel has ended
+  if (ld_cg_u32(&w.cnt->steps_count) == 0) return;  // grid-uniform: the probe kernel has ended
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
   uint32_t seq = 0;
   huge_hist<Tr>(sc, w, gtid >> 5, gthreads >> 5);
@@ -389,7 +389,7 @@ template <class Tr>
 __global__ void __launch_bounds__(256, 4)
     k_mutations(TableView t, Scratch sc, Window<Tr> w, GridBarrier* bar,
                 const uint32_t* fused_epoch) {
-  extern __shared__ uint32_t smem[];
+  extern __shared__ __align__(16) uint32_t smem[];
   const uint32_t f = ld_cg_u32(fused_epoch);
   w.epoch = 2 * dev_window_slot(fused_epoch) + 1;
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(256, 4)
   phase_probe_list<Tr>(t, sc, w, warp, nwarps, false);
   if (!grid_barrier(bar, gridDim.x, t.status, seq)) return;
   phase_sort_big<Tr>(sc, w, smem);
-  if (huge_groups(sc, w.cnt) == 0) return;  // grid-uniform: the probe step has ended
+  if (ld_cg_u32(&w.cnt->steps_count) == 0) return;  // grid-uniform: the probe step has ended
   huge_hist<Tr>(sc, w, gtid >> 5, gthreads >> 5);
   if (!grid_barrier(bar, gridDim.x, t.status, seq)) return;
   huge_scan<Tr>(sc, w, smem);
@@ -554,7 +554,7 @@ __device__ void fused_windows(const TableView& t, const Scratch& sc, const Fused
     // skips below are grid-uniform
     const bool has_big = ld_cg_u32(&w.cnt->big_count) != 0;
     const bool has_mut = ld_cg_u32(&w.cnt->mut_count) != 0;
-    const bool has_huge = huge_groups(sc, w.cnt) != 0;
+    const bool has_huge = ld_cg_u32(&w.cnt->steps_count) != 0;
     if (has_big || split < w.n) {
       if (has_big) phase_sort_big<Tr>(sc, w, smem);
       if (has_huge) huge_hist<Tr>(sc, w, warp, nwarps);
@@ -616,7 +616,7 @@ __device__ void fused_windows(const TableView& t, const Scratch& sc, const Fused
 template <class Tr, int P>
 __global__ void LSB_FUSED_BOUNDS
     k_fused(TableView t, Scratch sc, FusedJob<Tr> job, GridBarrier* bar) {
-  extern __shared__ uint32_t smem[];
+  extern __shared__ __align__(16) uint32_t smem[];
   uint32_t seq = 0;
   fused_windows<Tr, P>(t, sc, job, bar, smem, seq);
   release_counters(sc.cnt, bar, job.bins, 2 * sizeof(BinCounters) / 4);
@@ -872,7 +872,7 @@ struct AdmitNext {
 template <int P>
 __global__ void __launch_bounds__(1024, 1)
     k_serve(TableView t, Scratch sc, ServeJob j, GridBarrier* bar) {
-  extern __shared__ uint32_t smem[];
+  extern __shared__ __align__(16) uint32_t smem[];
   // spread indices (tid < 32 is still warp 0 of block 0)
   const uint32_t tid = spread_tid(), nt = gridDim.x * blockDim.x;
   uint32_t seq = 0;

@@ -40,13 +40,25 @@ constexpr uint32_t kPredLast = 0x80000000u;
 constexpr uint32_t kPredMask = 0x7FFFFFFFu;  // predecessor op index + 1; 0 = none
 constexpr uint32_t kWarpSort = 64;    // groups up to this size are ordered by one warp
 constexpr uint32_t kSortSmall = 4096;  // members a shared-memory sort holds
-// groups of more than kHugeMin members are ordered by many blocks (the huge_*
-// steps); smaller big groups by one block or one warp
+// larger groups are ordered by one block each, groups of more than kHugeMin
+// members by several, each taking an index range (sort_ranges), and groups of
+// more than kHugeSteps by the huge_* steps between grid barriers
 constexpr uint32_t kHugeMin = 4096;
-constexpr uint32_t kSortChunkWords = 2048;  // bitmap words per counting-sort pass
-// shared memory of the sort: kSortSmall members + kSortSmall sorted + bitmap
-// + prefix words
-constexpr uint32_t kSortSmemBytes = (2 * kSortSmall + 2 * kSortChunkWords) * 4;
+constexpr uint32_t kHugeSteps = 1u << 17;
+constexpr uint32_t kRangeMembers = 1024;  // mean members of a range
+// the shared-memory sort: members rank themselves against all others up to
+// kRankAll, in a bitmap of the index range where that is at most
+// kBitWords * 32 wide, and by counting into kSortBins ranges otherwise
+constexpr uint32_t kRankAll = 256;
+constexpr uint32_t kBitWords = 2048;
+constexpr uint32_t kSortBins = 4096;  // index ranges of the shared-memory sort
+// shared memory of the sort: members, members by range, range counts
+constexpr uint32_t kSortSmemBytes = (2 * kSortSmall + kSortBins + kSortBins / 32) * 4;
+// Word of range b: one word of padding per 32, so that threads scanning 4, 8
+// or 16 consecutive ranges each touch different banks (unpadded, 16 ranges
+// a thread were 16-way conflicts: 15 against 10 us for the ordering of a
+// 52k-put window).
+__host__ __device__ constexpr uint32_t bin_word(uint32_t b) { return b + (b >> 5); }
 
 // Group-table slot: bits 0..23 owner (op index + 1), 24..47 count, 48..63 epoch.
 __device__ __forceinline__ uint32_t g_owner(uint64_t v) { return (uint32_t)(v & 0xFFFFFFu); }
@@ -67,7 +79,8 @@ struct WinCounters {
   uint32_t huge_count;     // groups with more than kHugeMin members
   uint32_t run_count;      // runs of huge groups (each sorted by one block)
   uint32_t upd_count;      // updates among the window's mutations
-  uint32_t pad[4];
+  uint32_t steps_count;    // groups with more than kHugeSteps members
+  uint32_t pad[3];
 };
 
 __device__ inline void win_counters_reset(WinCounters* c) {
@@ -83,6 +96,7 @@ __device__ inline void win_counters_reset(WinCounters* c) {
   c->huge_count = 0;
   c->run_count = 0;
   c->upd_count = 0;
+  c->steps_count = 0;
 }
 
 // Scratch owned by a table, sized for max_window ops.
@@ -294,6 +308,7 @@ __device__ __forceinline__ void group_store(const Scratch& sc, const Window<Tr>&
       const uint32_t h = atomicAdd(&w.cnt->huge_count, 1u);
       if (h < sc.hcap) sc.hlist[h] = slot;
     }
+    if (pos == kHugeSteps) atomicAdd(&w.cnt->steps_count, 1u);
   }
 }
 
@@ -815,95 +830,142 @@ __device__ void block_lnu(const Scratch& sc, const Window<Tr>& w, const uint32_t
   __syncthreads();
 }
 
-// Counting sort of op indices by a bitmap over their range [lo, hi], in
-// passes of kSortChunkWords words; `get(j)` yields member j (< w.n) or an
-// out-of-range value to skip.  Writes the sorted list to seg[off ..].
-template <class Tr, class Get>
-__device__ void bitmap_sort(const Scratch& sc, const Window<Tr>& w, uint32_t c, uint32_t off,
-                            uint32_t* bits, uint32_t* pre, Get get, uint32_t* sorted) {
-  __shared__ uint32_t s_lo, s_hi, s_tmp[32];
+// Order the op indices mem[0..c) (shared memory, c <= kSortSmall; values
+// >= n are holes) ascending, the holes (as 0xFFFFFFFF) last; every valid one
+// lies in [lo, hi] (lo > hi: none is valid).  Returns the ordered list (mem or
+// `sorted`, which holds kSortSmall words too).  Whole block; mem, lo and hi are
+// settled by a barrier before the call, and the list by one at its end.
+//
+// Three ways, by size and spread, since the phase is one block's latency:
+//  - few members: each counts the smaller ones among all others.  One pass,
+//    one barrier; four members a load (the phase on a 20k-op window with nine
+//    such groups: 5.1 us, with one-word loads 7.5);
+//  - a narrow index range: a bitmap of it, ranks from its prefix popcounts
+//    (2600 members of a 52k-op range 3.3 us at 256 threads, the counting
+//    sort 5.6);
+//  - otherwise counting into equal ranges of [lo, hi], then each member ranks
+//    itself against the few others of its range, so the cost follows the
+//    group's size and not the window's (a bitmap of the whole of a 2^20-op
+//    window took 16 passes: 118 us for the ordering of a window of the 80/15/5
+//    queue, 67 this way).  Ranges are at most 256 ops wide in such a window,
+//    which bounds the ranking for members packed into a few of them.
+__device__ inline const uint32_t* order_members(uint32_t n, uint32_t c, uint32_t lo, uint32_t hi,
+                                                uint32_t* mem, uint32_t* sorted,
+                                                uint32_t* bins) {
+  __shared__ uint32_t s_tmp[32];
   const uint32_t tid = threadIdx.x, nt = blockDim.x;
-  uint32_t lo = 0xFFFFFFFFu, hi = 0;
-  for (uint32_t j = tid; j < c; j += nt) {
-    const uint32_t x = get(j);
-    if (x >= w.n) continue;  // never stored: skip rather than index with it
-    lo = min(lo, x);
-    hi = max(hi, x);
-  }
-  lo = __reduce_min_sync(0xFFFFFFFFu, lo);
-  hi = __reduce_max_sync(0xFFFFFFFFu, hi);
-  if (tid == 0) {
-    s_lo = 0xFFFFFFFFu;
-    s_hi = 0;
-  }
-  __syncthreads();
-  if ((tid & 31) == 0) {
-    atomicMin(&s_lo, lo);
-    atomicMax(&s_hi, hi);
-  }
-  __syncthreads();
-  lo = s_lo;
-  hi = s_hi;
-  __syncthreads();
-  uint32_t rank_base = 0;
-  const uint32_t span = kSortChunkWords * 32;
-  for (uint32_t cl = lo; cl <= hi; cl += span) {
-    const uint32_t words = min(kSortChunkWords, ((hi - cl) >> 5) + 1);
-    for (uint32_t k = tid; k < words; k += nt) bits[k] = 0;
+  if (c <= kRankAll) {
+    // four members a load (every lane reads the same word: a broadcast)
+    if (tid < 4 && c + tid < ((c + 3) & ~3u)) mem[c + tid] = 0xFFFFFFFFu;
+    for (uint32_t j = tid; j < c; j += nt) sorted[j] = 0xFFFFFFFFu;
     __syncthreads();
+    const uint4* four = reinterpret_cast<const uint4*>(mem);
     for (uint32_t j = tid; j < c; j += nt) {
-      const uint32_t x = get(j);
-      if (x <= hi && x >= cl && x - cl < span) atomicOr(&bits[(x - cl) >> 5], 1u << ((x - cl) & 31));
+      const uint32_t x = mem[j];
+      uint32_t r = 0;
+#pragma unroll 4
+      for (uint32_t q = 0; q < (c + 3) / 4; ++q) {
+        const uint4 v = four[q];
+        r += (v.x < x) + (v.y < x) + (v.z < x) + (v.w < x);
+      }
+      if (x < n) sorted[r] = x;
     }
     __syncthreads();
-    const uint32_t per = (words + nt - 1) / nt;
-    const uint32_t w0 = tid * per;
-    uint32_t local = 0;
-    for (uint32_t k = 0; k < per; ++k)
-      if (w0 + k < words) local += __popc(bits[w0 + k]);
-    uint32_t total;
+    return sorted;
+  }
+  uint32_t total, local = 0;
+  if (lo <= hi && hi - lo < kBitWords * 32) {
+    uint32_t* pre = bins + kBitWords;
+    const uint32_t words = (hi - lo) / 32 + 1, per = (words + nt - 1) / nt, w0 = tid * per;
+    for (uint32_t k = tid; k < words; k += nt) bins[k] = 0;
+    __syncthreads();
+    for (uint32_t j = tid; j < c; j += nt) {
+      const uint32_t x = mem[j] - lo;
+      if (mem[j] < n) atomicOr(&bins[x >> 5], 1u << (x & 31));
+    }
+    __syncthreads();
+    for (uint32_t k = w0; k < min(w0 + per, words); ++k) local += __popc(bins[k]);
     uint32_t run = block_exclusive_scan(local, s_tmp, &total);
-    for (uint32_t k = 0; k < per; ++k) {
-      if (w0 + k < words) {
-        pre[w0 + k] = run;
-        run += __popc(bits[w0 + k]);
-      }
+    for (uint32_t k = w0; k < min(w0 + per, words); ++k) {
+      pre[k] = run;
+      run += __popc(bins[k]);
     }
     __syncthreads();
     for (uint32_t j = tid; j < c; j += nt) {
-      const uint32_t x = get(j);
-      if (x <= hi && x >= cl && x - cl < span) {
-        const uint32_t d = x - cl, wd = d >> 5;
-        const uint32_t r = rank_base + pre[wd] + __popc(bits[wd] & ((1u << (d & 31)) - 1u));
-        sc.seg[off + r] = x;
-        if (sorted) sorted[r] = x;
-      }
+      const uint32_t x = mem[j] - lo;
+      if (mem[j] < n)
+        sorted[pre[x >> 5] + __popc(bins[x >> 5] & ((1u << (x & 31)) - 1u))] = mem[j];
+      if (j >= total) sorted[j] = 0xFFFFFFFFu;
     }
-    rank_base += total;
     __syncthreads();
-    if (hi - cl < span) break;
+    return sorted;
   }
+  const uint32_t nb = c <= kSortBins / 4 ? kSortBins / 4 : kSortBins;
+  uint32_t sh = 0;
+  while (lo < hi && ((hi - lo) >> sh) >= nb) ++sh;
+  for (uint32_t k = tid; k < bin_word(nb); k += nt) bins[k] = 0;
+  __syncthreads();
+  for (uint32_t j = tid; j < c; j += nt) {
+    const uint32_t x = mem[j];
+    if (x < n) atomicAdd(&bins[bin_word((x - lo) >> sh)], 1u);
+  }
+  __syncthreads();
+  const uint32_t per = (nb + nt - 1) / nt, b0 = tid * per;
+  for (uint32_t k = b0; k < min(b0 + per, nb); ++k) local += bins[bin_word(k)];
+  uint32_t run = block_exclusive_scan(local, s_tmp, &total);
+  for (uint32_t k = b0; k < min(b0 + per, nb); ++k) {
+    const uint32_t m = bins[bin_word(k)];
+    bins[bin_word(k)] = run;  // the range's start; its end once its members are placed
+    run += m;
+  }
+  __syncthreads();
+  for (uint32_t j = tid; j < c; j += nt) {
+    const uint32_t x = mem[j];
+    if (x < n) sorted[atomicAdd(&bins[bin_word((x - lo) >> sh)], 1u)] = x;
+  }
+  __syncthreads();
+  for (uint32_t j = tid; j < c; j += nt) {
+    if (j >= total) {
+      mem[j] = 0xFFFFFFFFu;
+      continue;
+    }
+    const uint32_t x = sorted[j], b = (x - lo) >> sh;
+    const uint32_t s = b ? bins[bin_word(b - 1)] : 0u, e = bins[bin_word(b)];
+    uint32_t r = s;
+    for (uint32_t q = s; q < e; ++q) r += sorted[q] < x;
+    mem[r] = x;
+  }
+  __syncthreads();
+  return mem;
 }
 
 // A group of kWarpSort+1 .. kHugeMin members, ordered by the whole block.
 // The members are gathered into shared memory first (a warp per storage
 // unit: the inline part, then each 32-member chunk with one chunk-table
-// lookup), so the counting sort reads only shared memory.
+// lookup), so the sort reads only shared memory.
 template <class Tr>
 __device__ void sort_group_block(const Scratch& sc, const Window<Tr>& w, uint32_t gslot,
                                  uint32_t c, uint32_t off, uint32_t* smem, bool upd) {
+  __shared__ uint32_t s_lo, s_hi;
   uint32_t* sorted = smem + kSortSmall;
-  uint32_t* bits = sorted + kSortSmall;
-  uint32_t* pre = bits + kSortChunkWords;
-  if (c > kSortSmall) return;  // block-uniform; larger groups take the huge_* phases
+  if (c > kSortSmall) return;  // block-uniform
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   const uint32_t nchunks = (c - kInline + kChunk - 1) / kChunk;  // <= kSortSmall / kChunk
   // all chunk-table lookups in flight at once (one per thread), parked in
-  // the prefix area; then each warp copies its chunks, loads issued before
-  // any store so they overlap
-  for (uint32_t k = tid; k < nchunks; k += blockDim.x) pre[k] = chunk_find(sc, w.epoch, gslot, k);
-  if (tid < kInline) smem[tid] = ld_cg_u32(&sc.ginl[(size_t)gslot * kInline + tid]);
-  for (uint32_t j = tid; j < c; j += blockDim.x) sorted[j] = 0xFFFFFFFFu;  // holes stay invalid
+  // the area of the sorted members; then each warp copies its chunks, loads
+  // issued before any store so they overlap
+  for (uint32_t k = tid; k < nchunks; k += blockDim.x)
+    sorted[k] = chunk_find(sc, w.epoch, gslot, k);
+  uint32_t lo = 0xFFFFFFFFu, hi = 0;
+  if (tid < kInline) {
+    const uint32_t x = ld_cg_u32(&sc.ginl[(size_t)gslot * kInline + tid]);
+    smem[tid] = x;
+    if (x < w.n) lo = hi = x;
+  }
+  if (tid == 0) {
+    s_lo = 0xFFFFFFFFu;
+    s_hi = 0;
+  }
   __syncthreads();
   for (uint32_t k0 = warp; k0 < nchunks; k0 += 4 * nwarps) {
     uint32_t v[4];
@@ -911,7 +973,7 @@ __device__ void sort_group_block(const Scratch& sc, const Window<Tr>& w, uint32_
     for (int q = 0; q < 4; ++q) {
       const uint32_t k = k0 + q * nwarps;
       const uint32_t j = kInline + k * kChunk + lane;
-      const uint32_t cs = k < nchunks ? pre[k] : 0xFFFFFFFFu;
+      const uint32_t cs = k < nchunks ? sorted[k] : 0xFFFFFFFFu;
       v[q] = (j < c && cs != 0xFFFFFFFFu) ? ld_cg_u32(&sc.cdat[(size_t)cs * kChunk + lane])
                                           : 0xFFFFFFFFu;
     }
@@ -919,104 +981,262 @@ __device__ void sort_group_block(const Scratch& sc, const Window<Tr>& w, uint32_
     for (int q = 0; q < 4; ++q) {
       const uint32_t j = kInline + (k0 + q * nwarps) * kChunk + lane;
       if (j < c) smem[j] = v[q];
-    }
-  }
-  __syncthreads();
-  bitmap_sort<Tr>(sc, w, c, off, bits, pre, [&](uint32_t j) { return smem[j]; }, sorted);
-  // every member's predecessor from the sorted list in shared memory (the
-  // bitmap pass ends with a __syncthreads)
-  for (uint32_t j = tid; j < c; j += blockDim.x) {
-    const uint32_t e = sorted[j];
-    const uint32_t pe = j ? sorted[j - 1] : 0xFFFFFFFFu;
-    const uint32_t p = pe < w.n ? pe + 1 : 0u;
-    if (e < w.n) sc.pred[e] = p | (j + 1 == c ? kPredLast : 0u);
-  }
-  __syncthreads();
-  if (upd) block_lnu<Tr>(sc, w, sorted, c, 0u);
-}
-
-// A group of kInline+1 .. kWarpSort members, ordered by one warp: each lane
-// holds members lane + 32h (h < K) and ranks them against all others by
-// shuffles, tracking each one's predecessor (the largest smaller index) on
-// the way (32 K^2 compares a lane).
-template <class Tr, int K>
-__device__ void sort_group_warp_k(const Scratch& sc, const Window<Tr>& w, uint32_t gslot,
-                                  uint32_t c, uint32_t off, bool upd) {
-  const uint32_t lane = lane_id();
-  uint32_t x[K];
-#pragma unroll
-  for (int h = 0; h < K; ++h) {
-    const uint32_t j = lane + 32 * h;
-    x[h] = j < c ? member_at(sc, w.epoch, gslot, j) : 0xFFFFFFFFu;
-  }
-  uint32_t rank[K], pred[K];
-#pragma unroll
-  for (int g = 0; g < K; ++g) {
-    rank[g] = 0;
-    pred[g] = 0xFFFFFFFFu;
-  }
-#pragma unroll
-  for (int h = 0; h < K; ++h) {
-    if (32u * h >= c) break;  // warp-uniform
-    for (uint32_t q = 0; q < 32; ++q) {
-      const uint32_t y = __shfl_sync(0xFFFFFFFFu, x[h], q);
-#pragma unroll
-      for (int g = 0; g < K; ++g) {
-        if (32 * h + q < c && y < x[g]) {
-          ++rank[g];
-          if (pred[g] == 0xFFFFFFFFu || y > pred[g]) pred[g] = y;
-        }
+      if (v[q] < w.n) {
+        lo = min(lo, v[q]);
+        hi = max(hi, v[q]);
       }
     }
   }
-#pragma unroll
-  for (int g = 0; g < K; ++g) {
-    const uint32_t j = lane + 32 * g;
-    if (j < c && x[g] < w.n) {
-      sc.seg[off + rank[g]] = x[g];
-      sc.pred[x[g]] = (pred[g] < w.n ? pred[g] + 1 : 0u) | (rank[g] + 1 == c ? kPredLast : 0u);
+  lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+  hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+  if (lane == 0) {
+    atomicMin(&s_lo, lo);
+    atomicMax(&s_hi, hi);
+  }
+  __syncthreads();
+  const uint32_t* list = order_members(w.n, c, s_lo, s_hi, smem, sorted, sorted + kSortSmall);
+  // the list, and every member's predecessor from it
+  for (uint32_t j = tid; j < c; j += blockDim.x) {
+    const uint32_t e = list[j];
+    const uint32_t pe = j ? list[j - 1] : 0xFFFFFFFFu;
+    if (e < w.n) {
+      sc.seg[off + j] = e;
+      sc.pred[e] = (pe < w.n ? pe + 1 : 0u) | (j + 1 == c ? kPredLast : 0u);
     }
   }
-  if (!upd) return;  // warp-uniform
-  // lnu: the largest smaller member that is not an update
-  uint32_t nu_of[K];
-#pragma unroll
-  for (int h = 0; h < K; ++h)
-    nu_of[h] = (x[h] < w.n && op_type(w, x[h]) != kOpUpdate) ? x[h] : 0xFFFFFFFFu;
-  uint32_t lnu[K];
-#pragma unroll
-  for (int g = 0; g < K; ++g) lnu[g] = 0;  // 1 + member, 0 = none
-#pragma unroll
-  for (int h = 0; h < K; ++h) {
-    if (32u * h >= c) break;  // warp-uniform
-    for (uint32_t q = 0; q < 32; ++q) {
-      const uint32_t y = __shfl_sync(0xFFFFFFFFu, nu_of[h], q);
-#pragma unroll
-      for (int g = 0; g < K; ++g)
-        if (y != 0xFFFFFFFFu && y < x[g] && y + 1 > lnu[g]) lnu[g] = y + 1;
-    }
-  }
-#pragma unroll
-  for (int g = 0; g < K; ++g)
-    if (lane + 32 * g < c && x[g] < w.n) sc.lnu[x[g]] = lnu[g];
+  __syncthreads();
+  if (upd) block_lnu<Tr>(sc, w, list, c, 0u);
 }
 
-// Two members a lane: groups of up to 64.  (Four a lane, groups up to 128
-// with the block sort taking only larger ones, measured slower: the fused
-// kernel spilled more at its 64-register cap, 97 -> 103 us on the 2^20-op
-// 95/5 batch, and the serving loop's latency did not change.)
+// A group of kInline+1 .. 32 K members, ordered by one warp in registers: a
+// bitonic sort of K members a lane (position 32 k + lane holds the k-th of
+// lane's; holes sort last), after which a member's predecessor is the one
+// before it and its last non-update predecessor a max-scan.  15 exchange
+// steps for 32 members and 21 for 64, against 32 K^2 compares a lane for
+// ranking each against all others (8 a lane, for groups of up to 256, measured
+// slower than a block each: 6 us for the one warp's 36 steps).  seg's space is taken with one atomic whose answer is first needed
+// for the stores.  The exchange loops stay rolled: the code runs once or twice a
+// launch, and unrolled its instruction fetches cost more than they save.
+template <class Tr, int K>
+__device__ __forceinline__ void sort_group_warp(const Scratch& sc, const Window<Tr>& w,
+                                             uint32_t gslot, uint32_t c, bool upd) {
+  const uint32_t lane = lane_id();
+  uint32_t off = 0, cs = 0xFFFFFFFFu;
+  if (lane == 0) off = atomicAdd(&w.cnt->seg_cursor, c);
+  // chunk k fills row k; the last row's chunk holds at most 24 members, which
+  // leaves its last lanes to the inline members
+  if (lane < (uint32_t)K && lane * kChunk + kInline < c) cs = chunk_find(sc, w.epoch, gslot, lane);
+  uint32_t x[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const uint32_t s = __shfl_sync(0xFFFFFFFFu, cs, k);
+    const uint32_t* from = &sc.cdat[(size_t)s * kChunk + lane];
+    bool in = kInline + k * kChunk + lane < c && s != 0xFFFFFFFFu;
+    if (k == K - 1 && lane >= kChunk - kInline) {
+      from = &sc.ginl[(size_t)gslot * kInline + lane - (kChunk - kInline)];
+      in = true;
+    }
+    x[k] = in ? ld_cg_u32(from) : 0xFFFFFFFFu;
+  }
+#pragma unroll 1
+  for (uint32_t size = 2; size <= 32 * K; size <<= 1) {
+#pragma unroll
+    for (uint32_t d = K / 2; d > 0; d >>= 1) {  // strides of 32 d: both members in this lane
+      if (size < 64 * d) continue;
+#pragma unroll
+      for (uint32_t k = 0; k < K; ++k) {
+        if (k & d) continue;
+        const uint32_t lo = min(x[k], x[k + d]), hi = max(x[k], x[k + d]);
+        const bool up = ((32 * k) & size) == 0;
+        x[k] = up ? lo : hi;
+        x[k + d] = up ? hi : lo;
+      }
+    }
+#pragma unroll 1
+    for (uint32_t stride = min(size >> 1, 16u); stride > 0; stride >>= 1) {
+#pragma unroll
+      for (uint32_t k = 0; k < K; ++k) {
+        const uint32_t y = __shfl_sync(0xFFFFFFFFu, x[k], lane ^ stride);
+        const bool low = ((lane & stride) == 0) == (((32 * k + lane) & size) == 0);
+        x[k] = low ? min(x[k], y) : max(x[k], y);
+      }
+    }
+  }
+  off = __shfl_sync(0xFFFFFFFFu, off, 0);
+  if (lane == 0) sc.goff[gslot] = off;
+  uint32_t before = 0, nu_before = 0;  // 1 + the member (non-update member) ending the last row
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const uint32_t j = lane + 32 * k, v = x[k] < w.n ? x[k] + 1 : 0u;  // 1 + member
+    uint32_t p = __shfl_up_sync(0xFFFFFFFFu, v, 1);
+    if (lane == 0) p = before;
+    before = __shfl_sync(0xFFFFFFFFu, v, 31);
+    if (j < c && v) {
+      sc.seg[off + j] = x[k];
+      sc.pred[x[k]] = p | (j + 1 == c ? kPredLast : 0u);
+    }
+    if (upd) {  // warp-uniform; members ascend, so the last is the largest
+      uint32_t m = (v && op_type(w, x[k]) != kOpUpdate) ? v : 0u;
+#pragma unroll
+      for (uint32_t d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, m, d);
+        if (lane >= d) m = max(m, y);
+      }
+      m = max(m, nu_before);
+      uint32_t e = __shfl_up_sync(0xFFFFFFFFu, m, 1);
+      if (lane == 0) e = nu_before;
+      nu_before = __shfl_sync(0xFFFFFFFFu, m, 31);
+      if (j < c && v) sc.lnu[x[k]] = e;
+    }
+  }
+}
+
+__device__ __forceinline__ uint32_t huge_groups(const Scratch& sc, const WinCounters* c) {
+  return min(ld_cg_u32(&c->huge_count), sc.hcap);
+}
+
+// Members of group gslot (c of them) with lo <= index < hi, in any order, into
+// mem[0..kSortSmall); *cnt their number (it may exceed kSortSmall; the surplus
+// is not stored), *below the number of members under lo, *prev and *carry
+// 1 + the largest of those and 1 + the largest that is not an update (0 =
+// none; carry only with upd).  Whole block; the four are shared variables.
 template <class Tr>
-__device__ void sort_group_warp(const Scratch& sc, const Window<Tr>& w, uint32_t gslot, uint32_t c,
-                                uint32_t off, bool upd) {
-  static_assert(kWarpSort == 64, "one warp holds at most 2 members a lane");
-  sort_group_warp_k<Tr, 2>(sc, w, gslot, c, off, upd);
+__device__ void gather_range(const Scratch& sc, const Window<Tr>& w, uint32_t gslot, uint32_t c,
+                             uint32_t lo, uint32_t hi, bool upd, uint32_t* mem,
+                             uint32_t* places, uint32_t* cnt, uint32_t* below, uint32_t* prev,
+                             uint32_t* carry) {
+  constexpr uint32_t kUnits = 8;  // chunks a warp reads at a time
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  // every chunk's place first (kHugeSteps / kChunk of them fit `places`), so
+  // that the chunk loads depend on nothing but shared memory
+  const uint32_t nchunks = (c - kInline + kChunk - 1) / kChunk;
+  for (uint32_t k = tid; k < nchunks; k += blockDim.x)
+    places[k] = chunk_find(sc, w.epoch, gslot, k);
+  if (tid == 0) *cnt = *below = *prev = *carry = 0;
+  __syncthreads();
+  uint32_t my_below = 0, my_prev = 0, my_carry = 0;
+  auto take = [&](uint32_t x) {  // whole warp
+    const bool in = x < w.n && x >= lo && x < hi;
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, in);
+    if (m) {
+      uint32_t at = 0;
+      if (lane == (uint32_t)__ffs(m) - 1) at = atomicAdd(cnt, (uint32_t)__popc(m));
+      at = __shfl_sync(0xFFFFFFFFu, at, __ffs(m) - 1) + __popc(m & ((1u << lane) - 1u));
+      if (in && at < kSortSmall) mem[at] = x;
+    }
+    if (x < lo) {
+      ++my_below;
+      my_prev = max(my_prev, x + 1);
+      if (upd && x + 1 > my_carry && op_type(w, x) != kOpUpdate) my_carry = x + 1;
+    }
+  };
+  if (warp == 0)
+    take(lane < kInline ? ld_cg_u32(&sc.ginl[(size_t)gslot * kInline + lane]) : 0xFFFFFFFFu);
+  for (uint32_t k0 = warp * kUnits; k0 < nchunks; k0 += nwarps * kUnits) {
+    uint32_t x[kUnits];
+#pragma unroll
+    for (uint32_t q = 0; q < kUnits; ++q) {
+      const uint32_t s = k0 + q < nchunks ? places[k0 + q] : 0xFFFFFFFFu;
+      const uint32_t j = kInline + (k0 + q) * kChunk + lane;
+      x[q] = (j < c && s != 0xFFFFFFFFu) ? ld_cg_u32(&sc.cdat[(size_t)s * kChunk + lane])
+                                         : 0xFFFFFFFFu;
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < kUnits; ++q) take(x[q]);
+  }
+  my_below = __reduce_add_sync(0xFFFFFFFFu, my_below);
+  my_prev = __reduce_max_sync(0xFFFFFFFFu, my_prev);
+  my_carry = __reduce_max_sync(0xFFFFFFFFu, my_carry);
+  if (lane == 0) {
+    atomicAdd(below, my_below);
+    atomicMax(prev, my_prev);
+    atomicMax(carry, my_carry);
+  }
+  __syncthreads();
+}
+
+// Members of group gslot (c of them) with lo <= index < end, ordered by the
+// whole block: their part of the group's list at seg[off ..) and their
+// predecessors.
+template <class Tr>
+__device__ void sort_range(const Scratch& sc, const Window<Tr>& w, uint32_t gslot, uint32_t c,
+                           uint32_t off, uint32_t lo, uint32_t end, bool upd, uint32_t* smem) {
+  __shared__ uint32_t s_cnt, s_below, s_prev, s_carry;
+  uint32_t* sorted = smem + kSortSmall;
+  uint32_t hi = end;
+  while (lo < end) {
+    gather_range<Tr>(sc, w, gslot, c, lo, hi, upd, smem, sorted + kSortSmall, &s_cnt, &s_below,
+                     &s_prev, &s_carry);
+    const uint32_t cnt = s_cnt, below = s_below, prev = s_prev, carry = s_carry;
+    if (cnt > kSortSmall) {  // members crowd here: as many indices as surely fit
+      hi = lo + kSortSmall;
+      __syncthreads();  // the counts are cleared again
+      continue;
+    }
+    const uint32_t* list = order_members(w.n, cnt, lo, hi - 1, smem, sorted, sorted + kSortSmall);
+    for (uint32_t j = threadIdx.x; j < cnt; j += blockDim.x) {
+      const uint32_t x = list[j], p = j ? list[j - 1] + 1 : prev;
+      if (x < w.n && below + j < c) {
+        sc.seg[off + below + j] = x;
+        sc.pred[x] = p | (below + j + 1 == c ? kPredLast : 0u);
+      }
+    }
+    __syncthreads();
+    if (upd) block_lnu<Tr>(sc, w, list, cnt, carry);
+    lo = hi;
+    hi = end;
+  }
+}
+
+// Groups of kHugeMin+1 .. kHugeSteps members (hot keys).  The window's indices
+// from its first mutation on are cut into equal ranges of about kRangeMembers
+// members, one job each; a block reads the whole group for its range, so it
+// knows the range's place in the group's list and the member before it, and no
+// block waits for another.  Reading the group once per range is cheap while it
+// is at most half a MB in L2, and it replaces four grid steps with barriers
+// between them (ordering of a window of the 80/15/5 queue 67 -> 39 us).  Jobs go to blocks by a static stride that starts behind
+// the blocks with a group of their own.  The lists fill seg from its end (other
+// groups from its start: all lists together hold at most max_window members).
+template <class Tr>
+__device__ void sort_ranges(const Scratch& sc, const Window<Tr>& w, uint32_t* smem, uint32_t job0,
+                            bool upd) {
+  const uint32_t lane = threadIdx.x & 31, g = gridDim.x;
+  // no mutation lies before it (0 when it was not recorded)
+  const uint32_t inv = ld_cg_u32(&w.cnt->inv_first_mut), first = inv ? ~inv : 0u;
+  const uint32_t H = huge_groups(sc, w.cnt);
+  if (first >= w.n) return;
+  uint32_t job = job0 % g, used = 0;  // jobs and seg entries of the groups before
+  for (uint32_t h0 = 0; h0 < H; h0 += 32) {
+    uint32_t gs = 0, cs = 0;  // lane l: group h0 + l
+    if (h0 + lane < H) {
+      gs = ld_cg_u32(&sc.hlist[h0 + lane]) & sc.gmask;
+      cs = min(g_count(ld_relaxed_u64(&sc.gtab[gs])), w.n);
+      if (cs > kHugeSteps || cs <= kHugeMin) cs = 0;
+    }
+    for (uint32_t q = 0; q < 32; ++q) {
+      const uint32_t c = __shfl_sync(0xFFFFFFFFu, cs, q);
+      const uint32_t gslot = __shfl_sync(0xFFFFFFFFu, gs, q);
+      if (c == 0) continue;  // grid-uniform, as is all that follows from c
+      used += c;
+      if (used > sc.max_window) return;  // cannot happen: members are distinct ops
+      const uint32_t off = sc.max_window - used;
+      const uint32_t ranges = (c + kRangeMembers - 1) / kRangeMembers;
+      const uint32_t width = (w.n - first + ranges - 1) / ranges;
+      for (uint32_t r = (blockIdx.x + g - job) % g; r < ranges; r += g) {
+        if (r == 0 && threadIdx.x == 0) sc.goff[gslot] = off;
+        sort_range<Tr>(sc, w, gslot, c, off, first + r * width, min(w.n, first + (r + 1) * width),
+                       upd, smem);
+      }
+      job = (job + ranges) % g;
+    }
+  }
 }
 
 // Phase D: block b orders large groups b, b + gridDim.x, ... (the critical
-// path); then warps take the groups of the big list by a static stride that
-// starts at the warps of blocks without a large group.  No work is claimed
-// through a shared counter, so no grid-wide atomic serializes the phase.
-// `smem` holds kSortSmemBytes.
+// path), then index ranges of hot keys; then warps take the groups of the big
+// list by a static stride that starts at the warps of blocks without a large
+// group.  No work is claimed through a shared counter, so no grid-wide atomic
+// serializes the phase.  `smem` holds kSortSmemBytes.
 template <class Tr>
 __device__ void phase_sort_big(const Scratch& sc, const Window<Tr>& w, uint32_t* smem) {
   __shared__ uint32_t s_off;
@@ -1026,7 +1246,7 @@ __device__ void phase_sort_big(const Scratch& sc, const Window<Tr>& w, uint32_t*
   for (uint32_t job = blockIdx.x; job < nlarge; job += gridDim.x) {
     const uint32_t gslot = ld_cg_u32(&sc.large[job]) & sc.gmask;
     const uint32_t c = min(g_count(ld_relaxed_u64(&sc.gtab[gslot])), w.n);
-    if (c > kHugeMin) continue;  // the huge_* steps order it (c is block-uniform)
+    if (c > kHugeMin) continue;  // ordered by many blocks (c is block-uniform)
     if (tid == 0) {
       s_off = atomicAdd(&w.cnt->seg_cursor, c);
       sc.goff[gslot] = s_off;
@@ -1035,8 +1255,9 @@ __device__ void phase_sort_big(const Scratch& sc, const Window<Tr>& w, uint32_t*
     const uint32_t off = s_off;
     sort_group_block<Tr>(sc, w, gslot, c, off, smem, upd);  // ends with __syncthreads
   }
+  if (ld_cg_u32(&w.cnt->huge_count)) sort_ranges<Tr>(sc, w, smem, nlarge, upd);
   const uint32_t nbig = ld_cg_u32(&w.cnt->big_count);
-  const uint32_t lane = lane_id(), wpb = blockDim.x >> 5;
+  const uint32_t wpb = blockDim.x >> 5;
   const uint32_t nw = gridDim.x * wpb;
   const uint32_t busy = min(nlarge, gridDim.x) * wpb;  // warps of blocks with a large group
   const uint32_t gw = blockIdx.x * wpb + (threadIdx.x >> 5);
@@ -1044,19 +1265,16 @@ __device__ void phase_sort_big(const Scratch& sc, const Window<Tr>& w, uint32_t*
     const uint32_t gslot = ld_cg_u32(&sc.big[job]) & sc.gmask;
     const uint32_t c = g_count(ld_relaxed_u64(&sc.gtab[gslot]));
     if (c > kWarpSort) continue;  // a block (or the huge steps) took it
-    uint32_t off = 0;
-    if (lane == 0) {
-      off = atomicAdd(&w.cnt->seg_cursor, c);
-      sc.goff[gslot] = off;
-    }
-    off = __shfl_sync(0xFFFFFFFFu, off, 0);
-    sort_group_warp<Tr>(sc, w, gslot, c, off, upd);
+    if (c <= 32)
+      sort_group_warp<Tr, 1>(sc, w, gslot, c, upd);
+    else
+      sort_group_warp<Tr, 2>(sc, w, gslot, c, upd);
   }
 }
 
 // ------------------------------------------------------- huge groups (D')
-// A group of more than kHugeMin members (a hot key) is ordered by the
-// whole grid in four steps separated by grid barriers, so no block reads
+// A group of more than kHugeSteps members (one key takes much of a window) is
+// ordered by the whole grid in four steps separated by grid barriers, so no block reads
 // back global data that it wrote itself in the same step:
 //   hist     every warp takes storage units (inline part / 32-member chunks)
 //            of every huge group and counts members per index range
@@ -1074,6 +1292,7 @@ __device__ void phase_sort_big(const Scratch& sc, const Window<Tr>& w, uint32_t*
 //            largest member for the first one).
 constexpr uint32_t kHugeBins = 4096;
 constexpr uint32_t kRunUnit = 2048;
+static_assert(kHugeSteps / kChunk <= kSortBins, "the chunk places of gather_range fit");
 static_assert(2 * kRunUnit == kSortSmall, "a run fits the shared-memory sort");
 constexpr uint32_t kRunFirst = 1u << 30, kRunLast = 1u << 31;
 
@@ -1081,9 +1300,6 @@ __device__ __forceinline__ uint32_t huge_width(uint32_t n) {
   return (n + kHugeBins - 1) / kHugeBins;  // <= kRunUnit for n <= 2^23
 }
 
-__device__ __forceinline__ uint32_t huge_groups(const Scratch& sc, const WinCounters* c) {
-  return min(ld_cg_u32(&c->huge_count), sc.hcap);
-}
 
 // Member `lane` of storage unit k of group gslot (unit 0: the inline part,
 // unit k >= 1: chunk k-1), or 0xFFFFFFFF.  Whole warp.
@@ -1116,6 +1332,7 @@ __device__ void huge_hist(const Scratch& sc, const Window<Tr>& w, uint32_t gwarp
   for (uint32_t h = 0; h < H; ++h) {
     uint32_t gslot;
     const uint32_t c = huge_size(sc, w, h, &gslot);
+    if (c <= kHugeSteps) continue;  // sort_ranges ordered it
     const uint32_t units = 1 + (c - kInline + kChunk - 1) / kChunk;
     uint32_t* bins = sc.hbins + (size_t)h * kHugeBins;
     for (uint32_t k = gwarp; k < units; k += ngwarps) {
@@ -1142,6 +1359,7 @@ __device__ void huge_scan(const Scratch& sc, const Window<Tr>& w, uint32_t* smem
     __syncthreads();
     uint32_t gslot;
     const uint32_t c = huge_size(sc, w, h, &gslot);
+    if (c <= kHugeSteps) continue;  // block-uniform
     uint32_t* bins = sc.hbins + (size_t)h * kHugeBins;
     uint32_t* hrun = sc.hrun + (size_t)h * kHugeBins;
     uint32_t local = 0;
@@ -1216,6 +1434,7 @@ __device__ void huge_scatter(const Scratch& sc, const Window<Tr>& w, uint32_t gw
   for (uint32_t h = 0; h < H; ++h) {
     uint32_t gslot;
     const uint32_t c = huge_size(sc, w, h, &gslot);
+    if (c <= kHugeSteps) continue;  // sort_group_ranges ordered it
     const uint32_t units = 1 + (c - kInline + kChunk - 1) / kChunk;
     uint32_t* bins = sc.hbins + (size_t)h * kHugeBins;
     const uint32_t* hrun = sc.hrun + (size_t)h * kHugeBins;
@@ -1256,9 +1475,8 @@ __device__ void huge_runs(const Scratch& sc, const Window<Tr>& w, uint32_t* smem
   const uint32_t R = min(ld_cg_u32(&w.cnt->run_count), sc.rcap);
   const bool upd = ld_cg_u32(&w.cnt->upd_count) != 0;
   __shared__ uint32_t s_carry;
+  __shared__ uint32_t s_lo, s_hi;
   uint32_t* sorted = smem + kSortSmall;
-  uint32_t* bits = sorted + kSortSmall;
-  uint32_t* pre = bits + kSortChunkWords;
   for (uint32_t r = blockIdx.x; r < R; r += gridDim.x) {
     const uint4 rec = ld_cg_v4(&sc.runs[4 * (size_t)r]);
     const uint32_t s = rec.x, e = rec.y, info = rec.z;
@@ -1267,19 +1485,38 @@ __device__ void huge_runs(const Scratch& sc, const Window<Tr>& w, uint32_t* smem
       n = e - s;
     else if (tid == 0)
       raise_status(sc.status, kStatusScratch);
+    if (tid == 0) {
+      s_lo = 0xFFFFFFFFu;
+      s_hi = 0;
+    }
+    uint32_t lo = 0xFFFFFFFFu, hi = 0;
     for (uint32_t j = tid; j < n; j += nt) {
-      smem[j] = ld_cg_u32(&sc.seg[s + j]);
-      sorted[j] = 0xFFFFFFFFu;
+      const uint32_t x = ld_cg_u32(&sc.seg[s + j]);
+      smem[j] = x;
+      if (x < w.n) {
+        lo = min(lo, x);
+        hi = max(hi, x);
+      }
+    }
+    lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+    hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+    __syncthreads();
+    if ((tid & 31) == 0) {
+      atomicMin(&s_lo, lo);
+      atomicMax(&s_hi, hi);
     }
     __syncthreads();
-    if (n) bitmap_sort<Tr>(sc, w, n, s, bits, pre, [&](uint32_t j) { return smem[j]; }, sorted);
+    const uint32_t* list = order_members(w.n, n, s_lo, s_hi, smem, sorted, sorted + kSortSmall);
     uint32_t first_pred = 0xFFFFFFFFu;
     if (!(info & kRunFirst) && r > 0) first_pred = ld_cg_u32(&sc.runs[4 * (size_t)(r - 1) + 3]) - 1u;
     for (uint32_t j = tid; j < n; j += nt) {
-      const uint32_t x = sorted[j];
-      const uint32_t pe = j ? sorted[j - 1] : first_pred;
+      const uint32_t x = list[j];
+      const uint32_t pe = j ? list[j - 1] : first_pred;
       const bool last = (info & kRunLast) && j + 1 == n;
-      if (x < w.n) sc.pred[x] = (pe < w.n ? pe + 1 : 0u) | (last ? kPredLast : 0u);
+      if (x < w.n) {
+        sc.seg[s + j] = x;
+        sc.pred[x] = (pe < w.n ? pe + 1 : 0u) | (last ? kPredLast : 0u);
+      }
     }
     __syncthreads();
     if (upd) {  // block-uniform
@@ -1296,7 +1533,7 @@ __device__ void huge_runs(const Scratch& sc, const Window<Tr>& w, uint32_t* smem
         s_carry = carry;
       }
       __syncthreads();
-      block_lnu<Tr>(sc, w, sorted, n, s_carry);  // ends with __syncthreads
+      block_lnu<Tr>(sc, w, list, n, s_carry);  // ends with __syncthreads
     }
   }
 }

@@ -1,0 +1,51 @@
+"""GPU parity of mixed batches whose groups sit on both sides of the ordering
+paths' limits (one warp, one block, index ranges over several blocks, grid
+steps) and spread over narrow and wide parts of the window: every result equals
+the oracle's replay, through the per-phase and the persistent form."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from lslab_b200 import Map
+from lslab_b200 import workload as W
+from oracle import OracleMap
+from tests.util import dev, first_mismatch, results, results_buf, same_results
+
+pytestmark = pytest.mark.gpu
+
+
+def _batch(kind):
+    rng = np.random.default_rng(41)
+    n = 1 << 19
+    t = np.zeros(n, np.uint8)
+    k = W.key_of_rank(6, rng.integers(0, 5000, size=n))
+    # 256 | 257 and 4096 | 4097 change the block's sort, 131072 | 131073 takes
+    # the grid steps
+    sizes = {"wide": (64, 65, 256, 257, 300, 4096, 4097, 9000, 131_072, 131_073),
+             "narrow": (64, 65, 256, 257, 1000, 4096, 4097, 20_000),
+             "many": (70,) * 3000 + (4200,) * 3}[kind]
+    at = rng.permutation(n) if kind != "narrow" else n - 1 - rng.permutation(60_000)
+    for i, c in enumerate(sizes):
+        m, at = at[:c], at[c:]
+        t[m], k[m] = rng.choice([1, 2, 3], size=c, p=[0.3, 0.2, 0.5]), np.uint64(10 + i)
+        # reads of the same key between its mutations
+        r = at[:c // 8]
+        at = at[c // 8:]
+        k[r] = np.uint64(10 + i)
+    return t, k, W.splitmix64(8, 0, n)
+
+
+@pytest.mark.parametrize("fused", [False, True])
+@pytest.mark.parametrize("kind", ["wide", "narrow", "many"])
+def test_group_sizes_at_path_limits(cuda, kind, fused):
+    import torch
+    t, k, v = _batch(kind)
+    m, o = Map(10), OracleMap(10)
+    for _ in range(2):  # the second time the keys that stayed are present
+        out = results_buf(len(k))
+        (m.execute_fused if fused else m.execute)(dev(t), dev(k), dev(v), out)
+        torch.cuda.synchronize()
+        got, want = results(out), o.mixed(t, k, v)
+        assert same_results(got, want), first_mismatch(got, want)
+    assert m.status() == 0
