@@ -24,11 +24,12 @@ namespace {
 constexpr uint32_t kDefaultWindow = 1u << 20;
 constexpr uint32_t kMaxWindow = 1u << 23;  // owner field of a group slot is 24 bits
 constexpr uint32_t kTraceCap = 1024;        // phase-trace entries per fused launch
-constexpr uint32_t kFusedEpochs = 32767;    // odd epochs 1..65535 for fused windows
-constexpr uint32_t kPlainEpochs = 32767;    // even epochs 2..65534 for per-phase windows
+constexpr uint32_t kFusedEpochs = kEpochs;  // odd epochs 1..253 for fused windows
+constexpr uint32_t kPlainEpochs = kEpochs;  // even epochs 2..254 for per-phase windows
+constexpr uint32_t kMaxFusedWindows = 16383;  // of one launch
 // One allocation for everything a fused launch zeroes first: two window
 // counter sets, the grid barrier, two region-counter sets.
-constexpr size_t kBinsOffset = 256;
+constexpr size_t kBinsOffset = 2304;
 constexpr size_t kCounterBytes = kBinsOffset + 2 * sizeof(BinCounters);
 static_assert(2 * sizeof(WinCounters) + sizeof(GridBarrier) <= kBinsOffset, "counter block");
 
@@ -343,7 +344,7 @@ __global__ void __launch_bounds__(1024, 1)
   extern __shared__ __align__(16) uint32_t smem[];
   if (fused_epoch != nullptr) w.epoch = 2 * dev_window_slot(fused_epoch) + 1;
   phase_sort_big<Tr>(sc, w, smem);
-  if (ld_cg_u32(&w.cnt->steps_count) == 0) return;  // grid-uniform: the probe kernel has ended
+  if (ld_settled(&w.cnt->steps_count) == 0) return;  // grid-uniform: the probe kernel has ended
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
   uint32_t seq = 0;
   huge_hist<Tr>(sc, w, gtid >> 5, gthreads >> 5);
@@ -374,7 +375,7 @@ template <class Tr>
 __global__ void __launch_bounds__(256, 4)
     k_probe_list(TableView t, Scratch sc, Window<Tr> w, const uint32_t* fused_epoch) {
   w.epoch = 2 * dev_window_slot(fused_epoch) + 1;
-  phase_probe_list<Tr>(t, sc, w, spread_warp(), (gridDim.x * blockDim.x) >> 5, false);
+  phase_probe_list<Tr>(t, sc, w, spread_warp(), (gridDim.x * blockDim.x) >> 5, false, false);
 }
 
 // The mutation steps of a window whose reads run beside it in k_read (the
@@ -401,10 +402,10 @@ __global__ void __launch_bounds__(256, 4)
   }
   phase_list_muts<Tr>(sc, w, warp, nwarps);
   if (!grid_barrier(bar, gridDim.x, t.status, seq)) return;
-  phase_probe_list<Tr>(t, sc, w, warp, nwarps, false);
+  phase_probe_list<Tr>(t, sc, w, warp, nwarps, false, false);
   if (!grid_barrier(bar, gridDim.x, t.status, seq)) return;
   phase_sort_big<Tr>(sc, w, smem);
-  if (ld_cg_u32(&w.cnt->steps_count) == 0) return;  // grid-uniform: the probe step has ended
+  if (ld_settled(&w.cnt->steps_count) == 0) return;  // grid-uniform: the probe step has ended
   huge_hist<Tr>(sc, w, gtid >> 5, gthreads >> 5);
   if (!grid_barrier(bar, gridDim.x, t.status, seq)) return;
   huge_scan<Tr>(sc, w, smem);
@@ -477,15 +478,16 @@ __device__ void fused_windows(const TableView& t, const Scratch& sc, const Fused
   // Window epochs live on the device so that a replayed CUDA graph of this
   // launch never reuses one: the fused path takes odd epochs 2f+1 (f = fused
   // windows so far), the per-phase path even ones from the host.  When the
-  // 16-bit epoch would wrap, the grid clears the group and chunk tables first.
-  uint32_t f = ld_cg_u32(job.fused_epoch);
-  if (f + nwin > kFusedEpochs) {
-    for (size_t i = tid; i <= sc.gmask; i += nt) sc.gtab[i] = 0;
-    for (size_t i = tid; i <= sc.cmask; i += nt) sc.ctab[i] = 0;
-    f = 0;
-    if (!grid_barrier(bar, nblocks, t.status, seq)) return;
-  }
-  for (uint32_t wi = 0; wi < nwin; ++wi) {
+  // epochs run out, the grid clears the group and chunk tables first.
+  const uint32_t f0 = ld_cg_u32(job.fused_epoch);
+  uint32_t f = f0;  // windows since the tables were cleared
+  for (uint32_t wi = 0; wi < nwin; ++wi, ++f) {
+    if (f + 1 > kFusedEpochs) {  // grid-uniform; the previous window has ended
+      for (size_t i = tid; i <= sc.gmask; i += nt) sc.gtab[i] = 0;
+      for (size_t i = tid; i <= sc.cmask; i += nt) sc.ctab[i] = 0;
+      f = 0;
+      if (!grid_barrier(bar, nblocks, t.status, seq)) return;
+    }
     trace_mark(job.trace, tat, wi, 0);
     Window<Tr> w = job.base;
     const uint32_t start = wi * job.window;
@@ -496,7 +498,7 @@ __device__ void fused_windows(const TableView& t, const Scratch& sc, const Fused
       w.vals = reinterpret_cast<const uint64_t*>(reinterpret_cast<const uint8_t*>(w.vals) +
                                                  (size_t)start * w.vstride * (w.v32 ? 4 : 8));
     if (w.out) w.out = (uint8_t*)w.out + (size_t)start * out_bytes(w.out_kind);
-    w.epoch = 2 * (f + wi) + 1;
+    w.epoch = 2 * f + 1;
     w.cnt = &sc.cnt[wi & 1];
     // the other counter sets were last read in window wi-1, which has ended
     if (tid == 0) win_counters_reset(&sc.cnt[(wi + 1) & 1]);
@@ -548,13 +550,13 @@ __device__ void fused_windows(const TableView& t, const Scratch& sc, const Fused
     }
     if (!grid_barrier(bar, nblocks, t.status, seq)) return;
     // every block has read the epoch counter (before its first barrier)
-    if (wi == 0 && tid == 0) *job.fused_epoch = f + nwin;
+    if (wi == 0 && tid == 0) *job.fused_epoch = (f0 + nwin - 1) % kFusedEpochs + 1;
     trace_mark(job.trace, tat, wi, 1);
     // counters read after the barrier: the same values in every block, so the
     // skips below are grid-uniform
-    const bool has_big = ld_cg_u32(&w.cnt->big_count) != 0;
-    const bool has_mut = ld_cg_u32(&w.cnt->mut_count) != 0;
-    const bool has_huge = ld_cg_u32(&w.cnt->steps_count) != 0;
+    const bool has_big = ld_settled(&w.cnt->big_count) != 0;
+    const bool has_mut = ld_settled(&w.cnt->inv_first_mut) != 0;
+    const bool has_huge = ld_settled(&w.cnt->steps_count) != 0;
     if (has_big || split < w.n) {
       if (has_big) phase_sort_big<Tr>(sc, w, smem);
       if (has_huge) huge_hist<Tr>(sc, w, warp, nwarps);
@@ -586,10 +588,11 @@ __device__ void fused_windows(const TableView& t, const Scratch& sc, const Fused
       // it pays one latency chain instead of two; a large one runs them one
       // after the other on the whole grid (mutations cost more per item).
       const uint32_t rt = tid - r0, rn = nt - r0;
-      const uint64_t m = ld_cg_u32(&w.cnt->mut_count);
-      const uint32_t first = ~ld_cg_u32(&w.cnt->inv_first_mut);
+      uint32_t len;
+      const uint64_t m = 32ull * __shfl_sync(0xFFFFFFFFu, mut_tiles(w, lane_id(), &len), 31);
+      const uint32_t first = ~ld_settled(&w.cnt->inv_first_mut);
       const uint64_t r = first < w.n ? w.n - first - 1 : 0;
-      const uint32_t ms = (uint32_t)((m + 31) / 32 * 32);
+      const uint32_t ms = (uint32_t)m;
       if (m + r + 32 <= rn) {
         if (rt < ms)
           phase_resolve_mutations<Tr>(t, sc, w, rt, ms);
@@ -1541,7 +1544,7 @@ struct Table {
     job.bin_shift = log2 > kBinBits ? log2 - kBinBits : 0u;
     if (trace) LSB_CK(cudaMemsetAsync(trace, 0, sizeof(uint64_t) * kTraceCap, s));
     uint32_t nwin = (uint32_t)((n + job.window - 1) / job.window);
-    if (nwin > kFusedEpochs / 2) return LSB_ERR_ARG;
+    if (nwin > kMaxFusedWindows) return LSB_ERR_ARG;
     const int grid = fused_grid();
     if (grid <= 0) return LSB_ERR_STATE;
     job.fused_epoch = fused_epoch;

@@ -34,6 +34,17 @@
 
 namespace lsb {
 
+// Loads of window scratch and counters that an earlier phase wrote and that
+// nothing writes any more, cached in L1 (a kernel boundary, or the acquire of
+// the grid barrier before the phase, keeps older lines out).  Words that every
+// warp of the grid looks at (counters, a hot key's group slot, list and owner
+// key) otherwise queue at the one L2 slice that holds them: the reads' resolve
+// of a window of the 80/15/5 queue took 93 us through L2 and 45 this way.
+template <class T>
+__device__ __forceinline__ T ld_settled(const T* p) {
+  return *p;
+}
+
 constexpr uint32_t kInline = 8;        // group members stored inline
 constexpr uint32_t kChunk = 32;        // members per overflow chunk
 constexpr uint32_t kPredLast = 0x80000000u;
@@ -60,14 +71,31 @@ constexpr uint32_t kSortSmemBytes = (2 * kSortSmall + kSortBins + kSortBins / 32
 // 52k-put window).
 __host__ __device__ constexpr uint32_t bin_word(uint32_t b) { return b + (b >> 5); }
 
-// Group-table slot: bits 0..23 owner (op index + 1), 24..47 count, 48..63 epoch.
+// Group-table slot: bits 0..23 owner (op index + 1), 24..47 count, 48..55 bits
+// of the key's hash, 56..63 epoch.  The hash bits keep a lookup from loading
+// the owner's key of a slot that holds another key (at most one group of other
+// keys in 256 costs a load), which is worth clearing the table every
+// kEpochs windows (16 MB for 2^20-op windows: 3 us in 127 windows).
 __device__ __forceinline__ uint32_t g_owner(uint64_t v) { return (uint32_t)(v & 0xFFFFFFu); }
 __device__ __forceinline__ uint32_t g_count(uint64_t v) { return (uint32_t)((v >> 24) & 0xFFFFFFu); }
-__device__ __forceinline__ uint32_t g_epoch(uint64_t v) { return (uint32_t)(v >> 48); }
+__device__ __forceinline__ uint32_t g_epoch(uint64_t v) { return (uint32_t)(v >> 56); }
+constexpr uint32_t kEpochs = 127;  // windows per parity (odd: persistent form, even: per-phase)
+
+// Epoch and hash bits of a key's group slot, as in bits 48..63.
+__device__ __forceinline__ uint32_t g_tag(uint32_t epoch, uint64_t h) {
+  return (epoch << 8) | (uint32_t)((h >> 12) & 0xFFu);
+}
+
+// The mutation list is kept in kMutSegs parts, part s for the ops of index
+// range s, each with a counter in a sector of its own: one counter that every
+// warp of the grid adds to is one L2 address that takes one atomic at a time
+// (probe of a 2^20-op window, half puts of uniform keys: 115 us with one, 106
+// with 32).
+constexpr uint32_t kMutSegs = 32;
+constexpr uint32_t kSegStride = 8;  // words between two counters
 
 // All counters start at zero, so a set is reset with a plain memset.
 struct WinCounters {
-  uint32_t mut_count;
   uint32_t seg_cursor;
   uint32_t big_count;
   uint32_t clist_count;    // entries of the compacted mutation list
@@ -80,11 +108,12 @@ struct WinCounters {
   uint32_t run_count;      // runs of huge groups (each sorted by one block)
   uint32_t upd_count;      // updates among the window's mutations
   uint32_t steps_count;    // groups with more than kHugeSteps members
-  uint32_t pad[3];
+  uint32_t pad[4];
+  uint32_t mut_seg[kMutSegs * kSegStride];  // mutations listed per index range
 };
 
 __device__ inline void win_counters_reset(WinCounters* c) {
-  c->mut_count = 0;
+  for (uint32_t k = 0; k < kMutSegs; ++k) c->mut_seg[k * kSegStride] = 0;
   c->seg_cursor = 0;
   c->big_count = 0;
   c->clist_count = 0;
@@ -160,7 +189,7 @@ struct Window {
   uint32_t kstride;      // elements between consecutive keys (2 for AoS pairs)
   uint32_t vstride;      // elements between consecutive values
   uint32_t n;
-  uint32_t epoch;        // 1..65535
+  uint32_t epoch;        // 1..255
   uint8_t uniform;
   uint8_t out_kind;
   uint8_t v32;           // values are 32-bit (stored zero-extended)
@@ -236,8 +265,18 @@ __device__ __forceinline__ uint32_t lane_id() {
 #endif
 }
 
+// First of the four group slots (one 32-byte sector) at which the search for a
+// key's group starts.
 __device__ __forceinline__ uint32_t gslot_of(uint64_t h, uint32_t gmask) {
-  return (uint32_t)(h >> 20) & gmask;
+  return (uint32_t)(h >> 20) & gmask & ~3u;
+}
+
+// Index ranges of the mutation list: op i is in range i >> seg_shift(n).  At
+// least 512 ops each, so that the ops of one list tile share one.
+__device__ __forceinline__ uint32_t seg_shift(uint32_t n) {
+  uint32_t sh = 9;
+  while (((n - 1) >> sh) >= kMutSegs) ++sh;
+  return sh;
 }
 
 // --------------------------------------------------------- overflow chunks
@@ -320,8 +359,8 @@ __device__ __forceinline__ uint32_t group_join(const Scratch& sc, const Window<T
                                                typename Tr::Key key, uint64_t h, uint32_t cnt,
                                                uint32_t* pos_out) {
   uint32_t slot = gslot_of(h, sc.gmask);
-  const uint64_t mine =
-      ((uint64_t)w.epoch << 48) | ((uint64_t)cnt << 24) | (uint64_t)(i + 1);
+  const uint32_t tag = g_tag(w.epoch, h);
+  const uint64_t mine = ((uint64_t)tag << 48) | ((uint64_t)cnt << 24) | (uint64_t)(i + 1);
   for (uint32_t probe = 0; probe <= sc.gmask; ++probe) {
     uint64_t v = ld_relaxed_u64(&sc.gtab[slot]);
     while (g_epoch(v) != w.epoch) {  // stale slot: try to claim it
@@ -332,7 +371,7 @@ __device__ __forceinline__ uint32_t group_join(const Scratch& sc, const Window<T
       }
       v = prev;
     }
-    if (key_of(w, g_owner(v) - 1) == key) {
+    if ((uint32_t)(v >> 48) == tag && key_of(w, g_owner(v) - 1) == key) {
       *pos_out = g_count(atomicAdd((unsigned long long*)&sc.gtab[slot], (uint64_t)cnt << 24));
       return slot;
     }
@@ -341,6 +380,13 @@ __device__ __forceinline__ uint32_t group_join(const Scratch& sc, const Window<T
   *pos_out = 0xFFFFFFFFu;
   return 0;
 }
+
+// What a warp has already told the window's counters, so that it tells each
+// thing once and not per tile.
+struct WarpNotes {
+  uint32_t lowest = 0xFFFFFFFFu;  // lowest mutation index reported
+  bool upd = false;               // an update was reported
+};
 
 // One tile of phase A: ops base + j*32 + lane for j < P.  kGroup: mutations
 // join groups (false for read-only batches).  dedup: lanes of a warp that
@@ -361,8 +407,9 @@ __device__ __forceinline__ void probe_ops(const TableView& t, const Scratch& sc,
                                           const Window<Tr>& w, uint32_t lane, bool dedup,
                                           const uint32_t (&idx)[P], const uint8_t (&type)[P],
                                           const bool (&active)[P],
-                                          const typename Tr::Key (&key)[P]) {
+                                          const typename Tr::Key (&key)[P], WarpNotes& notes) {
   const uint32_t lanemask_lt = (1u << lane) - 1u;
+  const uint32_t sshift = seg_shift(w.n);
   uint64_t h[P], value[P], loc[P];
   bool want[P], found[P];
   uint32_t src[P];
@@ -408,15 +455,30 @@ __device__ __forceinline__ void probe_ops(const TableView& t, const Scratch& sc,
       const uint32_t mm = __ballot_sync(0xFFFFFFFFu, is_mut);
       if (mm) {
         const uint32_t first = __reduce_min_sync(0xFFFFFFFFu, is_mut ? i : 0xFFFFFFFFu);
-        uint32_t slot_base = 0;
-        const uint32_t ldr = __ffs(mm) - 1;
         const uint32_t um = __ballot_sync(0xFFFFFFFFu, is_mut && type[j] == kOpUpdate);
-        if (lane == ldr) {
-          slot_base = atomicAdd(&w.cnt->mut_count, (uint32_t)__popc(mm));
-          atomicMax(&w.cnt->inv_first_mut, ~first);
-          if (um) atomicAdd(&w.cnt->upd_count, (uint32_t)__popc(um));
+        if (first < notes.lowest) {
+          notes.lowest = first;
+          if (lane == 0) atomicMax(&w.cnt->inv_first_mut, ~first);
         }
-        slot_base = __shfl_sync(0xFFFFFFFFu, slot_base, ldr);
+        if (um && !notes.upd) {
+          notes.upd = true;
+          if (lane == 0) atomicAdd(&w.cnt->upd_count, 1u);
+        }
+        // a place in the list of each mutation's index range (one range,
+        // except in the region order, whose tiles mix ranges)
+        uint32_t place = 0;
+        for (uint32_t todo = mm; todo;) {
+          const uint32_t ldr = __ffs(todo) - 1;
+          const uint32_t seg = __shfl_sync(0xFFFFFFFFu, i >> sshift, ldr);
+          const uint32_t same = __ballot_sync(0xFFFFFFFFu, is_mut && i >> sshift == seg);
+          uint32_t base = 0;
+          if (lane == ldr)
+            base = (seg << sshift) +
+                   atomicAdd(&w.cnt->mut_seg[seg * kSegStride], (uint32_t)__popc(same));
+          base = __shfl_sync(0xFFFFFFFFu, base, ldr);
+          if (is_mut && i >> sshift == seg) place = base + __popc(same & lanemask_lt);
+          todo &= ~same;
+        }
         // same-key mutations of this warp join together: the lowest lane
         // (lowest op index) joins for all and hands out consecutive
         // positions in lane order, which is op-index order
@@ -428,7 +490,7 @@ __device__ __forceinline__ void probe_ops(const TableView& t, const Scratch& sc,
         gslot = __shfl_sync(0xFFFFFFFFu, gslot, lead);
         gpos = __shfl_sync(0xFFFFFFFFu, gpos, lead);
         if (is_mut) {
-          sc.mlist[slot_base + __popc(mm & lanemask_lt)] = i;
+          if (place < sc.max_window) sc.mlist[place] = i;
           group_store<Tr>(sc, w, gslot, gpos + __popc(peers & lanemask_lt), i, loc[j]);
         }
       }
@@ -443,7 +505,7 @@ template <class Tr, bool kGroup, int P>
 __device__ __forceinline__ void probe_tile(const TableView& t, const Scratch& sc,
                                            const Window<Tr>& w, uint32_t base, uint32_t lane,
                                            bool dedup, const ProbeSel& sel,
-                                           const uint32_t* perm) {
+                                           const uint32_t* perm, WarpNotes& notes) {
   using Key = typename Tr::Key;
   Key key[P];
   uint8_t type[P];
@@ -459,7 +521,7 @@ __device__ __forceinline__ void probe_tile(const TableView& t, const Scratch& sc
     active[j] = i < w.n && (type[j] == kOpRead ? (pos >= sel.read_lo && pos < sel.read_hi) : sel.muts);
     key[j] = active[j] ? (perm ? key_of(w, i) : key_stream(w, i)) : (Key)0;
   }
-  probe_ops<Tr, kGroup, P>(t, sc, w, lane, dedup, idx, type, active, key);
+  probe_ops<Tr, kGroup, P>(t, sc, w, lane, dedup, idx, type, active, key, notes);
 }
 
 // Phase A for the mutations of a window (its reads are probed by blocks
@@ -527,9 +589,11 @@ __device__ void phase_list_muts(const Scratch& sc, const Window<Tr>& w, uint32_t
 
 template <class Tr>
 __device__ void phase_probe_list(const TableView& t, const Scratch& sc, const Window<Tr>& w,
-                                 uint32_t warp_id, uint32_t num_warps, bool dedup) {
+                                 uint32_t warp_id, uint32_t num_warps, bool dedup,
+                                 bool count_tiles = true) {
   using Key = typename Tr::Key;
   const uint32_t lane = lane_id();
+  WarpNotes notes;
   const uint32_t total = min(ld_cg_u32(&w.cnt->clist_count), clist_cap(sc.max_window));
   for (uint32_t tile = warp_id * 32; tile < total; tile += num_warps * 32) {
     const uint32_t i = tile + lane < total ? ld_cg_u32(sc.clist + tile + lane) : 0xFFFFFFFFu;
@@ -543,8 +607,9 @@ __device__ void phase_probe_list(const TableView& t, const Scratch& sc, const Wi
       active[0] = type[0] != kOpRead;
       key[0] = key_of(w, i);
     }
-    probe_ops<Tr, true, 1>(t, sc, w, lane, dedup, idx, type, active, key);
-    if (lane == 0) atomicAdd(&w.cnt->tiles_done, 1u);
+    probe_ops<Tr, true, 1>(t, sc, w, lane, dedup, idx, type, active, key, notes);
+    // (only blocks that read meanwhile watch the count)
+    if (count_tiles && lane == 0) atomicAdd(&w.cnt->tiles_done, 1u);
   }
 }
 
@@ -564,9 +629,10 @@ __device__ void phase_probe(const TableView& t, const Scratch& sc, const Window<
                             const uint32_t* perm = nullptr, const uint32_t* stop_at = nullptr,
                             uint32_t stop_target = 0) {
   const uint32_t lane = lane_id();
+  WarpNotes notes;
   if (cursor == nullptr || chunk == 0) {
     for (uint32_t base = begin + warp_id * 32 * P; base < w.n; base += num_warps * 32 * P)
-      probe_tile<Tr, kGroup, P>(t, sc, w, base, lane, dedup, sel, perm);
+      probe_tile<Tr, kGroup, P>(t, sc, w, base, lane, dedup, sel, perm, notes);
     return;
   }
   __shared__ uint32_t s_base, s_next;
@@ -590,7 +656,7 @@ __device__ void phase_probe(const TableView& t, const Scratch& sc, const Window<
       if (lane == 0) off = atomicAdd(&s_next, 32u * P);
       off = __shfl_sync(0xFFFFFFFFu, off, 0);
       if (c0 + off >= c1) break;
-      probe_tile<Tr, kGroup, P>(t, sc, w, c0 + off, lane, dedup, sel, perm);
+      probe_tile<Tr, kGroup, P>(t, sc, w, c0 + off, lane, dedup, sel, perm, notes);
     }
     __syncthreads();  // s_base / s_next are rewritten next round
   }
@@ -1092,7 +1158,7 @@ __device__ __forceinline__ void sort_group_warp(const Scratch& sc, const Window<
 }
 
 __device__ __forceinline__ uint32_t huge_groups(const Scratch& sc, const WinCounters* c) {
-  return min(ld_cg_u32(&c->huge_count), sc.hcap);
+  return min(ld_settled(&c->huge_count), sc.hcap);
 }
 
 // Members of group gslot (c of them) with lo <= index < hi, in any order, into
@@ -1202,7 +1268,7 @@ __device__ void sort_ranges(const Scratch& sc, const Window<Tr>& w, uint32_t* sm
                             bool upd) {
   const uint32_t lane = threadIdx.x & 31, g = gridDim.x;
   // no mutation lies before it (0 when it was not recorded)
-  const uint32_t inv = ld_cg_u32(&w.cnt->inv_first_mut), first = inv ? ~inv : 0u;
+  const uint32_t inv = ld_settled(&w.cnt->inv_first_mut), first = inv ? ~inv : 0u;
   const uint32_t H = huge_groups(sc, w.cnt);
   if (first >= w.n) return;
   uint32_t job = job0 % g, used = 0;  // jobs and seg entries of the groups before
@@ -1241,8 +1307,8 @@ template <class Tr>
 __device__ void phase_sort_big(const Scratch& sc, const Window<Tr>& w, uint32_t* smem) {
   __shared__ uint32_t s_off;
   const uint32_t tid = threadIdx.x;
-  const bool upd = ld_cg_u32(&w.cnt->upd_count) != 0;  // settled: the probe has ended
-  const uint32_t nlarge = ld_cg_u32(&w.cnt->large_count);
+  const bool upd = ld_settled(&w.cnt->upd_count) != 0;  // settled: the probe has ended
+  const uint32_t nlarge = ld_settled(&w.cnt->large_count);
   for (uint32_t job = blockIdx.x; job < nlarge; job += gridDim.x) {
     const uint32_t gslot = ld_cg_u32(&sc.large[job]) & sc.gmask;
     const uint32_t c = min(g_count(ld_relaxed_u64(&sc.gtab[gslot])), w.n);
@@ -1255,8 +1321,8 @@ __device__ void phase_sort_big(const Scratch& sc, const Window<Tr>& w, uint32_t*
     const uint32_t off = s_off;
     sort_group_block<Tr>(sc, w, gslot, c, off, smem, upd);  // ends with __syncthreads
   }
-  if (ld_cg_u32(&w.cnt->huge_count)) sort_ranges<Tr>(sc, w, smem, nlarge, upd);
-  const uint32_t nbig = ld_cg_u32(&w.cnt->big_count);
+  if (ld_settled(&w.cnt->huge_count)) sort_ranges<Tr>(sc, w, smem, nlarge, upd);
+  const uint32_t nbig = ld_settled(&w.cnt->big_count);
   const uint32_t wpb = blockDim.x >> 5;
   const uint32_t nw = gridDim.x * wpb;
   const uint32_t busy = min(nlarge, gridDim.x) * wpb;  // warps of blocks with a large group
@@ -1430,7 +1496,7 @@ template <class Tr>
 __device__ void huge_scatter(const Scratch& sc, const Window<Tr>& w, uint32_t gwarp,
                              uint32_t ngwarps) {
   const uint32_t H = huge_groups(sc, w.cnt), width = huge_width(w.n), lane = lane_id();
-  const bool upd = ld_cg_u32(&w.cnt->upd_count) != 0;
+  const bool upd = ld_settled(&w.cnt->upd_count) != 0;
   for (uint32_t h = 0; h < H; ++h) {
     uint32_t gslot;
     const uint32_t c = huge_size(sc, w, h, &gslot);
@@ -1472,8 +1538,8 @@ __device__ void huge_runs(const Scratch& sc, const Window<Tr>& w, uint32_t* smem
   const uint32_t tid = threadIdx.x, nt = blockDim.x;
   const uint32_t H = huge_groups(sc, w.cnt);
   for (size_t i = gtid; i < (size_t)H * kHugeBins; i += gthreads) sc.hbins[i] = 0;
-  const uint32_t R = min(ld_cg_u32(&w.cnt->run_count), sc.rcap);
-  const bool upd = ld_cg_u32(&w.cnt->upd_count) != 0;
+  const uint32_t R = min(ld_settled(&w.cnt->run_count), sc.rcap);
+  const bool upd = ld_settled(&w.cnt->upd_count) != 0;
   __shared__ uint32_t s_carry;
   __shared__ uint32_t s_lo, s_hi;
   uint32_t* sorted = smem + kSortSmall;
@@ -1577,7 +1643,7 @@ __device__ __noinline__ uint32_t inline_lnu(const Scratch& sc, const Window<Tr>&
                                             uint32_t c, uint32_t x) {
   uint32_t best = 0xFFFFFFFFu;
   for (uint32_t q = 0; q < c && q < kInline; ++q) {
-    const uint32_t m = ld_cg_u32(&sc.ginl[(size_t)gslot * kInline + q]);
+    const uint32_t m = ld_settled(&sc.ginl[(size_t)gslot * kInline + q]);
     if (m < x && m < w.n && (best == 0xFFFFFFFFu || m > best) && op_type(w, m) != kOpUpdate)
       best = m;
   }
@@ -1595,11 +1661,11 @@ __device__ __forceinline__ bool present_before(const Scratch& sc, const Window<T
   if (c <= kInline) {
     l = inline_lnu<Tr>(sc, w, gslot, c, x);
   } else {
-    const uint32_t e = ld_cg_u32(&sc.lnu[x]);
+    const uint32_t e = ld_settled(&sc.lnu[x]);
     l = e ? e - 1 : 0xFFFFFFFFu;
   }
   if (l < w.n) return op_type(w, l) == kOpWrite;
-  return (ld_cg_u64(&sc.mloc[x]) & kLocLive) != 0;
+  return (ld_settled(&sc.mloc[x]) & kLocLive) != 0;
 }
 
 // Post-state of mutation p (group gslot of c members) as (present, value):
@@ -1620,8 +1686,8 @@ __device__ __forceinline__ void post_state(const Scratch& sc, const Window<Tr>& 
 // whether i is the group's last mutation.
 __device__ __forceinline__ uint32_t inline_pred(const Scratch& sc, uint32_t gslot, uint32_t c,
                                                 uint32_t i, uint32_t n, bool* last) {
-  const uint4 a = ld_cg_v4(&sc.ginl[(size_t)gslot * kInline]);
-  const uint4 b = ld_cg_v4(&sc.ginl[(size_t)gslot * kInline + 4]);
+  const uint4 a = ld_settled(reinterpret_cast<const uint4*>(&sc.ginl[(size_t)gslot * kInline]));
+  const uint4 b = ld_settled(reinterpret_cast<const uint4*>(&sc.ginl[(size_t)gslot * kInline + 4]));
   const uint32_t m[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
   uint32_t best = 0xFFFFFFFFu;
   bool later = false;
@@ -1636,12 +1702,36 @@ __device__ __forceinline__ uint32_t inline_pred(const Scratch& sc, uint32_t gslo
   return best;
 }
 
+// Whole tiles of 32 in the parts of the mutation list up to part `lane`
+// (inclusive), and the part's length.  Whole warp.
+template <class Tr>
+__device__ __forceinline__ uint32_t mut_tiles(const Window<Tr>& w, uint32_t lane, uint32_t* len) {
+  static_assert(kMutSegs == 32, "a lane a part");
+  const uint32_t c = ld_settled(&w.cnt->mut_seg[lane * kSegStride]);
+  uint32_t t = (c + 31) / 32;
+#pragma unroll
+  for (uint32_t d = 1; d < 32; d <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, t, d);
+    if (lane >= d) t += y;
+  }
+  *len = c;
+  return t;
+}
+
+// Threads tid of nthreads, whole warps, take the list's tiles in turn.
 template <class Tr>
 __device__ void phase_resolve_mutations(const TableView& t, const Scratch& sc,
                                         const Window<Tr>& w, uint32_t tid, uint32_t nthreads) {
-  const uint32_t mcount = ld_cg_u32(&w.cnt->mut_count);
-  for (uint32_t j = tid; j < mcount; j += nthreads) {
-    const uint32_t m = ld_cg_u32(&sc.mlist[j]);
+  const uint32_t lane = tid & 31u, sshift = seg_shift(w.n);
+  uint32_t len;
+  const uint32_t upto = mut_tiles(w, lane, &len);
+  const uint32_t tiles = __shfl_sync(0xFFFFFFFFu, upto, 31);
+  for (uint32_t tile = tid >> 5; tile < tiles; tile += nthreads >> 5) {
+    const uint32_t seg = __popc(__ballot_sync(0xFFFFFFFFu, upto <= tile));
+    const uint32_t before = seg ? __shfl_sync(0xFFFFFFFFu, upto, (seg - 1) & 31u) : 0u;
+    const uint32_t at = (tile - before) * 32 + lane;
+    if (at >= __shfl_sync(0xFFFFFFFFu, len, seg & 31u)) continue;
+    const uint32_t m = ld_cg_u32(&sc.mlist[(seg << sshift) + at]);
     if (m >= w.n) continue;
     // everything that depends on m alone in one round trip: the group slot,
     // the op, the slot location its probe found and its ordering record
@@ -1652,7 +1742,7 @@ __device__ void phase_resolve_mutations(const TableView& t, const Scratch& sc,
     const uint8_t type = op_type(w, m);
     const typename Tr::Key key = key_of(w, m);
     const uint32_t gslot = (uint32_t)(mi >> 32) & sc.gmask;
-    const uint32_t c = g_count(ld_relaxed_u64(&sc.gtab[gslot]));
+    const uint32_t c = g_count(ld_settled(&sc.gtab[gslot]));
     uint32_t pred;
     bool last = true;
     if (c == 1) {
@@ -1681,7 +1771,7 @@ __device__ void phase_resolve_mutations(const TableView& t, const Scratch& sc,
 template <class Tr>
 __device__ void phase_resolve_reads(const Scratch& sc, const Window<Tr>& w, uint32_t tid,
                                     uint32_t nthreads) {
-  const uint32_t first = ~ld_cg_u32(&w.cnt->inv_first_mut);
+  const uint32_t first = ~ld_settled(&w.cnt->inv_first_mut);
   if (first >= w.n) return;
   for (uint32_t i = first + 1 + tid; i < w.n; i += nthreads) {
     const uint8_t type = op_type(w, i);
@@ -1689,16 +1779,25 @@ __device__ void phase_resolve_reads(const Scratch& sc, const Window<Tr>& w, uint
     const typename Tr::Key key = key_of(w, i);
     const uint64_t h = Tr::hash(key);
     uint32_t slot = gslot_of(h, sc.gmask);
+    const uint32_t tag = g_tag(w.epoch, h);
     uint64_t v = 0;
-    bool hit = false;
-    for (uint32_t probe = 0; probe <= sc.gmask; ++probe) {
-      v = ld_relaxed_u64(&sc.gtab[slot]);
-      if (g_epoch(v) != w.epoch) break;
-      if (key_of(w, g_owner(v) - 1) == key) {
-        hit = true;
-        break;
+    bool hit = false, end = false;
+    for (uint32_t probe = 0; probe <= sc.gmask && !end; probe += 4) {
+      const ulonglong2* four = reinterpret_cast<const ulonglong2*>(&sc.gtab[slot]);
+      const ulonglong2 v01 = ld_settled(four), v23 = ld_settled(four + 1);
+      const uint64_t vs[4] = {v01.x, v01.y, v23.x, v23.y};
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q) {
+        if (end) continue;
+        if (g_epoch(vs[q]) != w.epoch) {  // a free slot ends the search
+          end = true;
+        } else if ((uint32_t)(vs[q] >> 48) == tag && key_of(w, g_owner(vs[q]) - 1) == key) {
+          v = vs[q];
+          slot += q;
+          hit = end = true;
+        }
       }
-      slot = (slot + 1) & sc.gmask;
+      if (!end) slot = (slot + 4) & sc.gmask;
     }
     if (!hit) continue;
     const uint32_t c = g_count(v);
@@ -1707,17 +1806,17 @@ __device__ void phase_resolve_reads(const Scratch& sc, const Window<Tr>& w, uint
       bool last;
       pred_op = inline_pred(sc, slot, c, i, w.n, &last);
     } else {
-      const uint32_t off = ld_cg_u32(&sc.goff[slot]);
+      const uint32_t off = ld_settled(&sc.goff[slot]);
       if (off > sc.max_window || c > sc.max_window - off) continue;
       uint32_t lo = 0, hi = c;  // count of members < i
       while (lo < hi) {
         uint32_t mid = (lo + hi) >> 1;
-        if (ld_cg_u32(&sc.seg[off + mid]) < i)
+        if (ld_settled(&sc.seg[off + mid]) < i)
           lo = mid + 1;
         else
           hi = mid;
       }
-      if (lo > 0) pred_op = ld_cg_u32(&sc.seg[off + lo - 1]);
+      if (lo > 0) pred_op = ld_settled(&sc.seg[off + lo - 1]);
     }
     if (pred_op < w.n) {
       bool present;

@@ -49,3 +49,23 @@ def test_group_sizes_at_path_limits(cuda, kind, fused):
         got, want = results(out), o.mixed(t, k, v)
         assert same_results(got, want), first_mismatch(got, want)
     assert m.status() == 0
+
+
+@pytest.mark.parametrize("fused", [False, True])
+def test_many_windows_of_one_call(cuda, fused):
+    """One call of several hundred windows: the 127 window epochs run out within
+    the call, so the group tables are cleared between its windows."""
+    import torch
+    rng = np.random.default_rng(43)
+    n, window = 64 * 300 + 17, 64
+    t = rng.choice([0, 1, 2, 3], size=n, p=[0.4, 0.3, 0.1, 0.2]).astype(np.uint8)
+    k = W.key_of_rank(7, rng.integers(0, 50, size=n))
+    v = W.splitmix64(9, 0, n)
+    m, o = Map(6, max_window=window), OracleMap(6)
+    for _ in range(2):
+        out = results_buf(n)
+        (m.execute_fused if fused else m.execute)(dev(t), dev(k), dev(v), out)
+        torch.cuda.synchronize()
+        got, want = results(out), o.mixed(t, k, v)
+        assert same_results(got, want), first_mismatch(got, want)
+    assert m.status() == 0
