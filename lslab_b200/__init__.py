@@ -42,13 +42,16 @@ def _ptr(x) -> int | None:
         return None
     if isinstance(x, int):
         return x
-    if hasattr(x, "data_ptr"):
-        if not x.is_cuda:
-            raise ValueError("device buffers are required (got a CPU tensor)")
-        if not x.is_contiguous():
-            raise ValueError("buffers must be contiguous")
-        return x.data_ptr()
-    raise TypeError(f"expected a CUDA tensor or a device pointer, got {type(x).__name__}")
+    try:
+        ptr = x.data_ptr
+    except AttributeError:
+        raise TypeError(
+            f"expected a CUDA tensor or a device pointer, got {type(x).__name__}") from None
+    if not x.is_cuda:
+        raise ValueError("device buffers are required (got a CPU tensor)")
+    if not x.is_contiguous():
+        raise ValueError("buffers must be contiguous")
+    return ptr()
 
 
 def _len(x, size):
@@ -59,13 +62,35 @@ def _len(x, size):
     raise ValueError("size is required when passing raw pointers")
 
 
-def _stream(s) -> int | None:
-    if s is None:
+_raw_stream = None  # torch's current raw stream, as a function, once torch is in use
+
+
+def _current_stream() -> int | None:
+    """torch's current stream as a cudaStream_t (None without torch or a GPU).
+    Small calls are bound by the host, and building a torch.cuda.Stream only
+    to read its handle was a good part of one (a get of 500 keys: 8.9 us a
+    call, 4.8 with the raw handle and the bound functions below)."""
+    global _raw_stream
+    if _raw_stream is None:
         try:
             import torch
-            return torch.cuda.current_stream().cuda_stream
+            handle = torch.cuda.current_stream().cuda_stream  # initialises CUDA
+            get, device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+            if get(device()) == handle:
+                _raw_stream = lambda: get(device())  # noqa: E731
+            else:
+                _raw_stream = lambda: torch.cuda.current_stream().cuda_stream  # noqa: E731
+            return handle
+        except AttributeError:  # a torch without the raw accessors
+            _raw_stream = lambda: torch.cuda.current_stream().cuda_stream  # noqa: E731
         except Exception:
             return None
+    return _raw_stream()
+
+
+def _stream(s) -> int | None:
+    if s is None:
+        return _current_stream()
     if isinstance(s, int):
         return s
     return s.cuda_stream
@@ -93,9 +118,19 @@ class _Table:
         self._h = h
         self.n_log_2 = int(n_log_2)
 
+    _fns: dict = {}  # the container's C functions by name, bound on first use
+
+    def __init_subclass__(cls, **kw):
+        super().__init_subclass__(**kw)
+        cls._fns = {}
+
     def _call(self, name, *args):
-        _lib.check(getattr(lib(), f"lsb_{self._prefix}_{name}")(self._h, *args),
-                   f"lsb_{self._prefix}_{name}")
+        fn = self._fns.get(name)
+        if fn is None:
+            fn = self._fns[name] = getattr(lib(), f"lsb_{self._prefix}_{name}")
+        rc = fn(self._h, *args)
+        if rc:
+            _lib.check(rc, f"lsb_{self._prefix}_{name}")
 
     def device_view(self) -> dict:
         """The table's device handles (lsb_*_device_view): slab array pointer,
