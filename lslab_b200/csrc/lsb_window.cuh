@@ -1771,6 +1771,7 @@ __device__ void phase_resolve_mutations(const TableView& t, const Scratch& sc,
 template <class Tr>
 __device__ void phase_resolve_reads(const Scratch& sc, const Window<Tr>& w, uint32_t tid,
                                     uint32_t nthreads) {
+  if (w.types == nullptr && w.uniform != kOpRead) return;  // no reads
   const uint32_t first = ~ld_settled(&w.cnt->inv_first_mut);
   if (first >= w.n) return;
   for (uint32_t i = first + 1 + tid; i < w.n; i += nthreads) {
