@@ -482,13 +482,13 @@ __device__ __forceinline__ bool table_find(const TableView& t, typename Tr::Key 
   return find_rest<Tr>(t, key, rep, s, m.next, tag_match(m, rep), val, loc);
 }
 
-// The lean single lookup of the read-only paths (k_read, and the fused
-// kernel's read loop): the head meta sector, the first candidate slot inline,
-// the rest of the chain in find_rest.  Few registers: it runs in kernels
-// bounded to 32 a thread.
+// The lean single lookup (one op a thread): the head meta sector, the first
+// candidate slot inline, the rest of the chain in find_rest.  Few registers:
+// it runs in kernels bounded to 32 a thread.  *loc: where the key lives, as
+// find_rest reports it (0 when absent).
 template <class Tr>
-__device__ __forceinline__ bool read_lookup(const TableView& t, typename Tr::Key key,
-                                            uint64_t* val) {
+__device__ __forceinline__ bool lean_lookup(const TableView& t, typename Tr::Key key,
+                                            uint64_t* val, uint64_t* loc) {
   const uint64_t h = Tr::hash(key);
   const uint32_t s = (uint32_t)h & t.mask;
   const uint32_t rep = (0x80u | fingerprint(h)) * 0x01010101u;
@@ -496,10 +496,12 @@ __device__ __forceinline__ bool read_lookup(const TableView& t, typename Tr::Key
   const Meta m = load_meta<true>(slab);
   uint32_t cand = tag_match(m, rep);
   *val = 0;
+  *loc = 0;
   bool found = false;
   if (cand) {
     const int slot = __ffs(cand) - 1;
     cand &= cand - 1;
+    *loc = kLocLive | ((uint64_t)s << 8) | (uint64_t)slot;
     if constexpr (Tr::kHasValue) {
       const ulonglong2 kv = ld_ca_v2u64(slab + kMetaBytes + slot * Tr::kSlotBytes);
       found = kv.x == (uint64_t)key;
@@ -508,12 +510,21 @@ __device__ __forceinline__ bool read_lookup(const TableView& t, typename Tr::Key
       found = ld_ca_u32(slab + kMetaBytes + slot * Tr::kSlotBytes) == (uint32_t)key;
     }
   }
-  if (!found && (cand || m.next != 0)) {
-    uint64_t loc;
-    found = find_rest<Tr>(t, key, rep, s, m.next, cand, val, &loc);
-    if (!found) *val = 0;
+  if (!found) {
+    *loc = 0;
+    if (cand || m.next != 0) {
+      found = find_rest<Tr>(t, key, rep, s, m.next, cand, val, loc);
+      if (!found) *val = 0;
+    }
   }
   return found;
+}
+
+template <class Tr>
+__device__ __forceinline__ bool read_lookup(const TableView& t, typename Tr::Key key,
+                                            uint64_t* val) {
+  uint64_t loc;
+  return lean_lookup<Tr>(t, key, val, &loc);
 }
 
 // P independent lookups issued together: all head meta sectors first, then

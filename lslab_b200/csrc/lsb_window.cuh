@@ -265,10 +265,14 @@ __device__ __forceinline__ uint32_t lane_id() {
 #endif
 }
 
-// First of the four group slots (one 32-byte sector) at which the search for a
-// key's group starts.
+// The group slot at which the search for a key's group starts.  It goes on in
+// the other slots of the same four (one 32-byte sector), then in the next four:
+// a lookup reads four at a time, and as slots are never freed within a window,
+// a free one among them ends it.  (Joins all starting at the first of the four
+// would meet another key's group there more often: 2^20 puts of uniform keys
+// 248 us a call against 242.)
 __device__ __forceinline__ uint32_t gslot_of(uint64_t h, uint32_t gmask) {
-  return (uint32_t)(h >> 20) & gmask & ~3u;
+  return (uint32_t)(h >> 20) & gmask;
 }
 
 // Index ranges of the mutation list: op i is in range i >> seg_shift(n).  At
@@ -330,10 +334,9 @@ __device__ __forceinline__ uint32_t member_at(const Scratch& sc, uint32_t epoch,
 // ---------------------------------------------------------------- phase A
 // Store member i at position pos of group `slot` (inline or in a chunk).
 template <class Tr>
-__device__ __forceinline__ void group_store(const Scratch& sc, const Window<Tr>& w, uint32_t slot,
-                                            uint32_t pos, uint32_t i, uint64_t loc) {
+__device__ __forceinline__ void group_place(const Scratch& sc, const Window<Tr>& w, uint32_t slot,
+                                            uint32_t pos, uint32_t i) {
   sc.minfo[i] = ((uint64_t)slot << 32) | pos;
-  sc.mloc[i] = loc;
   if (pos >= sc.max_window) return;  // no group (cannot happen: the table has 2x room)
   if (pos < kInline) {
     sc.ginl[(size_t)slot * kInline + pos] = i;
@@ -351,6 +354,14 @@ __device__ __forceinline__ void group_store(const Scratch& sc, const Window<Tr>&
   }
 }
 
+// The same, with the slot that the probe found for the op.
+template <class Tr>
+__device__ __forceinline__ void group_store(const Scratch& sc, const Window<Tr>& w, uint32_t slot,
+                                            uint32_t pos, uint32_t i, uint64_t loc) {
+  sc.mloc[i] = loc;
+  group_place<Tr>(sc, w, slot, pos, i);
+}
+
 // Join `cnt` mutations of `key` (op indices carried by the caller's peer
 // lanes) to the key's group; returns the group slot and the position of the
 // first of them.  The group's owner (first joiner) claims the slot by CAS.
@@ -358,10 +369,12 @@ template <class Tr>
 __device__ __forceinline__ uint32_t group_join(const Scratch& sc, const Window<Tr>& w, uint32_t i,
                                                typename Tr::Key key, uint64_t h, uint32_t cnt,
                                                uint32_t* pos_out) {
-  uint32_t slot = gslot_of(h, sc.gmask);
+  const uint32_t start = gslot_of(h, sc.gmask);
   const uint32_t tag = g_tag(w.epoch, h);
   const uint64_t mine = ((uint64_t)tag << 48) | ((uint64_t)cnt << 24) | (uint64_t)(i + 1);
   for (uint32_t probe = 0; probe <= sc.gmask; ++probe) {
+    const uint32_t slot =
+        ((start + (probe & ~3u)) & sc.gmask & ~3u) | ((start + probe) & 3u);
     uint64_t v = ld_relaxed_u64(&sc.gtab[slot]);
     while (g_epoch(v) != w.epoch) {  // stale slot: try to claim it
       uint64_t prev = atomicCAS((unsigned long long*)&sc.gtab[slot], v, mine);
@@ -375,7 +388,6 @@ __device__ __forceinline__ uint32_t group_join(const Scratch& sc, const Window<T
       *pos_out = g_count(atomicAdd((unsigned long long*)&sc.gtab[slot], (uint64_t)cnt << 24));
       return slot;
     }
-    slot = (slot + 1) & sc.gmask;
   }
   *pos_out = 0xFFFFFFFFu;
   return 0;
@@ -387,6 +399,58 @@ struct WarpNotes {
   uint32_t lowest = 0xFFFFFFFFu;  // lowest mutation index reported
   bool upd = false;               // an update was reported
 };
+
+// The mutations among a warp's 32 ops (lane: op i) join their groups and the
+// mutation list.  loc: the op's slot from the probe, recorded too (null: the
+// lookups record it).  Whole warp; lanes in ascending op-index order.
+template <class Tr>
+__device__ __forceinline__ void group_tile(const Scratch& sc, const Window<Tr>& w, uint32_t lane,
+                                           uint32_t i, bool is_mut, uint8_t type,
+                                           typename Tr::Key key, uint64_t h, WarpNotes& notes,
+                                           const uint64_t* loc) {
+  const uint32_t mm = __ballot_sync(0xFFFFFFFFu, is_mut);
+  if (!mm) return;
+  const uint32_t lanemask_lt = (1u << lane) - 1u, sshift = seg_shift(w.n);
+  const uint32_t first = __reduce_min_sync(0xFFFFFFFFu, is_mut ? i : 0xFFFFFFFFu);
+  const uint32_t um = __ballot_sync(0xFFFFFFFFu, is_mut && type == kOpUpdate);
+  if (first < notes.lowest) {
+    notes.lowest = first;
+    if (lane == 0) atomicMax(&w.cnt->inv_first_mut, ~first);
+  }
+  if (um && !notes.upd) {
+    notes.upd = true;
+    if (lane == 0) atomicAdd(&w.cnt->upd_count, 1u);
+  }
+  // a place in the list of each mutation's index range (one range, except in
+  // the region order, whose tiles mix ranges)
+  uint32_t place = 0;
+  for (uint32_t todo = mm; todo;) {
+    const uint32_t ldr = __ffs(todo) - 1;
+    const uint32_t seg = __shfl_sync(0xFFFFFFFFu, i >> sshift, ldr);
+    const uint32_t same = __ballot_sync(0xFFFFFFFFu, is_mut && i >> sshift == seg);
+    uint32_t base = 0;
+    if (lane == ldr)
+      base = (seg << sshift) +
+             atomicAdd(&w.cnt->mut_seg[seg * kSegStride], (uint32_t)__popc(same));
+    base = __shfl_sync(0xFFFFFFFFu, base, ldr);
+    if (is_mut && i >> sshift == seg) place = base + __popc(same & lanemask_lt);
+    todo &= ~same;
+  }
+  // same-key mutations of this warp join together: the lowest lane (lowest op
+  // index) joins for all and hands out consecutive positions in lane order,
+  // which is op-index order
+  const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key) & mm;
+  const uint32_t lead = is_mut ? __ffs(peers) - 1 : lane;
+  uint32_t gslot = 0, gpos = 0;
+  if (is_mut && lead == lane) gslot = group_join<Tr>(sc, w, i, key, h, __popc(peers), &gpos);
+  gslot = __shfl_sync(0xFFFFFFFFu, gslot, lead);
+  gpos = __shfl_sync(0xFFFFFFFFu, gpos, lead);
+  if (is_mut) {
+    if (place < sc.max_window) sc.mlist[place] = i;
+    if (loc != nullptr) sc.mloc[i] = *loc;
+    group_place<Tr>(sc, w, gslot, gpos + __popc(peers & lanemask_lt), i);
+  }
+}
 
 // One tile of phase A: ops base + j*32 + lane for j < P.  kGroup: mutations
 // join groups (false for read-only batches).  dedup: lanes of a warp that
@@ -408,8 +472,6 @@ __device__ __forceinline__ void probe_ops(const TableView& t, const Scratch& sc,
                                           const uint32_t (&idx)[P], const uint8_t (&type)[P],
                                           const bool (&active)[P],
                                           const typename Tr::Key (&key)[P], WarpNotes& notes) {
-  const uint32_t lanemask_lt = (1u << lane) - 1u;
-  const uint32_t sshift = seg_shift(w.n);
   uint64_t h[P], value[P], loc[P];
   bool want[P], found[P];
   uint32_t src[P];
@@ -450,51 +512,9 @@ __device__ __forceinline__ void probe_ops(const TableView& t, const Scratch& sc,
     }
     const uint32_t i = idx[j];
     if (active[j]) write_result(w, i, type[j], found[j], value[j]);
-    if (kGroup) {
-      const bool is_mut = active[j] && type[j] != kOpRead;
-      const uint32_t mm = __ballot_sync(0xFFFFFFFFu, is_mut);
-      if (mm) {
-        const uint32_t first = __reduce_min_sync(0xFFFFFFFFu, is_mut ? i : 0xFFFFFFFFu);
-        const uint32_t um = __ballot_sync(0xFFFFFFFFu, is_mut && type[j] == kOpUpdate);
-        if (first < notes.lowest) {
-          notes.lowest = first;
-          if (lane == 0) atomicMax(&w.cnt->inv_first_mut, ~first);
-        }
-        if (um && !notes.upd) {
-          notes.upd = true;
-          if (lane == 0) atomicAdd(&w.cnt->upd_count, 1u);
-        }
-        // a place in the list of each mutation's index range (one range,
-        // except in the region order, whose tiles mix ranges)
-        uint32_t place = 0;
-        for (uint32_t todo = mm; todo;) {
-          const uint32_t ldr = __ffs(todo) - 1;
-          const uint32_t seg = __shfl_sync(0xFFFFFFFFu, i >> sshift, ldr);
-          const uint32_t same = __ballot_sync(0xFFFFFFFFu, is_mut && i >> sshift == seg);
-          uint32_t base = 0;
-          if (lane == ldr)
-            base = (seg << sshift) +
-                   atomicAdd(&w.cnt->mut_seg[seg * kSegStride], (uint32_t)__popc(same));
-          base = __shfl_sync(0xFFFFFFFFu, base, ldr);
-          if (is_mut && i >> sshift == seg) place = base + __popc(same & lanemask_lt);
-          todo &= ~same;
-        }
-        // same-key mutations of this warp join together: the lowest lane
-        // (lowest op index) joins for all and hands out consecutive
-        // positions in lane order, which is op-index order
-        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key[j]) & mm;
-        const uint32_t lead = is_mut ? __ffs(peers) - 1 : lane;
-        uint32_t gslot = 0, gpos = 0;
-        if (is_mut && lead == lane)
-          gslot = group_join<Tr>(sc, w, i, key[j], h[j], __popc(peers), &gpos);
-        gslot = __shfl_sync(0xFFFFFFFFu, gslot, lead);
-        gpos = __shfl_sync(0xFFFFFFFFu, gpos, lead);
-        if (is_mut) {
-          if (place < sc.max_window) sc.mlist[place] = i;
-          group_store<Tr>(sc, w, gslot, gpos + __popc(peers & lanemask_lt), i, loc[j]);
-        }
-      }
-    }
+    if (kGroup)
+      group_tile<Tr>(sc, w, lane, i, active[j] && type[j] != kOpRead, type[j], key[j], h[j], notes,
+                     &loc[j]);
   }
 }
 
@@ -659,6 +679,108 @@ __device__ void phase_probe(const TableView& t, const Scratch& sc, const Window<
       probe_tile<Tr, kGroup, P>(t, sc, w, c0 + off, lane, dedup, sel, perm, notes);
     }
     __syncthreads();  // s_base / s_next are rewritten next round
+  }
+}
+
+// Phase A as two kinds of work that need nothing of each other, so that warps
+// take them side by side: a lookup's round trips (meta sector, slot) go to the
+// table and are bound by random access to it, a join's (group slot, chunk)
+// stay in L2.  In one pass an op waits for both in turn, in a kernel of twice
+// the registers (probe of 777 puts 6.9 -> 4.5 us, six calls on a set 101 -> 88,
+// probe phase of a 20k-op window in the persistent kernel 11.6 -> 9.5).
+//
+// Lookups: thread tid of nthreads; every op's tentative result, and for
+// mutations the slot.
+template <class Tr>
+__device__ __forceinline__ void phase_lookup(const TableView& t, const Scratch& sc,
+                                             const Window<Tr>& w, uint32_t tid,
+                                             uint32_t nthreads) {
+  for (uint32_t i = tid; i < w.n; i += nthreads) {
+    const uint8_t type = op_type_stream(w, i);
+    uint64_t val, loc;
+    const bool found = lean_lookup<Tr>(t, key_stream(w, i), &val, &loc);
+    write_result(w, i, type, found, val);
+    if (type != kOpRead) sc.mloc[i] = loc;
+  }
+}
+
+__device__ __forceinline__ void warp_sync() {
+#ifdef LSB_HOST_EMU
+  __ballot_sync(0xFFFFFFFFu, true);
+#else
+  __syncwarp();
+#endif
+}
+
+// Joins: warp warp_id of num_warps takes spans of 32 ops.  When every warp has
+// one of 128 ops, it takes those instead and first packs their mutations, so
+// that the joins of a read-mostly mix run with full warps (and more same-key
+// ops share one); with fewer the packing would only leave warps idle.  `slice`
+// is kJoinSpan bytes of shared memory of the warp's own.
+constexpr uint32_t kJoinSpan = 128;
+
+template <class Tr>
+__device__ void phase_join(const Scratch& sc, const Window<Tr>& w, uint32_t warp_id,
+                           uint32_t num_warps, uint8_t* slice) {
+  using Key = typename Tr::Key;
+  if (w.types == nullptr && w.uniform == kOpRead) return;
+  const uint32_t lane = lane_id();
+  WarpNotes notes;
+  if (w.types == nullptr || w.n < kJoinSpan * num_warps) {
+    for (uint32_t base = warp_id * 32; base < w.n; base += num_warps * 32) {
+      const uint32_t i = base + lane;
+      const uint8_t type = i < w.n ? op_type(w, i) : (uint8_t)kOpRead;
+      const bool is_mut = type != kOpRead;
+      const Key key = is_mut ? key_of(w, i) : (Key)0;
+      group_tile<Tr>(sc, w, lane, i, is_mut, type, key, Tr::hash(key), notes, nullptr);
+    }
+    return;
+  }
+  constexpr uint32_t kPer = kJoinSpan / 32;
+  for (uint32_t base = warp_id * kJoinSpan; base < w.n; base += num_warps * kJoinSpan) {
+    uint32_t bits = 0;  // bit k: op base + kPer * lane + k is a mutation
+    for (uint32_t k = 0; k < kPer; ++k) {
+      const uint32_t i = base + kPer * lane + k;
+      if (i < w.n && op_type(w, i) != kOpRead) bits |= 1u << k;
+    }
+    uint32_t incl = __popc(bits);
+#pragma unroll
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+      if (lane >= d) incl += y;
+    }
+    const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    uint32_t at = incl - __popc(bits);
+    for (uint32_t m = bits; m; m &= m - 1u)
+      slice[at++] = (uint8_t)(kPer * lane + (uint32_t)(__ffs(m) - 1));
+    warp_sync();
+    for (uint32_t q = 0; q < total; q += 32) {
+      const bool is_mut = q + lane < total;
+      const uint32_t i = is_mut ? base + slice[q + lane] : 0u;
+      const uint8_t type = is_mut ? op_type(w, i) : (uint8_t)kOpRead;
+      const Key key = is_mut ? key_of(w, i) : (Key)0;
+      group_tile<Tr>(sc, w, lane, i, is_mut, type, key, Tr::hash(key), notes, nullptr);
+    }
+    warp_sync();  // the slice is written again
+  }
+}
+
+// The listed mutations (phase_list_muts) join their groups; their lookups run
+// elsewhere (the two-stream form's read kernel).
+template <class Tr>
+__device__ void phase_join_list(const Scratch& sc, const Window<Tr>& w, uint32_t warp_id,
+                                uint32_t num_warps) {
+  using Key = typename Tr::Key;
+  const uint32_t lane = lane_id();
+  WarpNotes notes;
+  const uint32_t total = min(ld_settled(&w.cnt->clist_count), clist_cap(sc.max_window));
+  for (uint32_t tile = warp_id * 32; tile < total; tile += num_warps * 32) {
+    uint32_t i = tile + lane < total ? ld_cg_u32(sc.clist + tile + lane) : 0xFFFFFFFFu;
+    const uint8_t type = i < w.n ? op_type(w, i) : (uint8_t)kOpRead;
+    const bool is_mut = type != kOpRead;
+    if (!is_mut) i = 0;
+    const Key key = is_mut ? key_of(w, i) : (Key)0;
+    group_tile<Tr>(sc, w, lane, i, is_mut, type, key, Tr::hash(key), notes, nullptr);
   }
 }
 
@@ -1779,7 +1901,7 @@ __device__ void phase_resolve_reads(const Scratch& sc, const Window<Tr>& w, uint
     if (type != kOpRead) continue;
     const typename Tr::Key key = key_of(w, i);
     const uint64_t h = Tr::hash(key);
-    uint32_t slot = gslot_of(h, sc.gmask);
+    uint32_t slot = gslot_of(h, sc.gmask) & ~3u;
     const uint32_t tag = g_tag(w.epoch, h);
     uint64_t v = 0;
     bool hit = false, end = false;
@@ -1787,18 +1909,18 @@ __device__ void phase_resolve_reads(const Scratch& sc, const Window<Tr>& w, uint
       const ulonglong2* four = reinterpret_cast<const ulonglong2*>(&sc.gtab[slot]);
       const ulonglong2 v01 = ld_settled(four), v23 = ld_settled(four + 1);
       const uint64_t vs[4] = {v01.x, v01.y, v23.x, v23.y};
+      uint32_t at = slot;
 #pragma unroll
       for (uint32_t q = 0; q < 4; ++q) {
-        if (end) continue;
-        if (g_epoch(vs[q]) != w.epoch) {  // a free slot ends the search
-          end = true;
-        } else if ((uint32_t)(vs[q] >> 48) == tag && key_of(w, g_owner(vs[q]) - 1) == key) {
+        end |= g_epoch(vs[q]) != w.epoch;
+        if (!hit && (uint32_t)(vs[q] >> 48) == tag && key_of(w, g_owner(vs[q]) - 1) == key) {
           v = vs[q];
-          slot += q;
-          hit = end = true;
+          at = slot + q;
+          hit = true;
         }
       }
-      if (!end) slot = (slot + 4) & sc.gmask;
+      end |= hit;
+      slot = hit ? at : (slot + 4) & sc.gmask;
     }
     if (!hit) continue;
     const uint32_t c = g_count(v);
