@@ -133,7 +133,9 @@ typedef struct lsb_tuning {
                              steps cost more than the locality saves) */
 } lsb_tuning;
 
-#define LSB_LOCK_WRITER 0u   /* writers take a per-bucket lock; readers never lock   */
+#define LSB_LOCK_WRITER 0u   /* readers never lock; the per-warp device API's writers take
+                                a per-bucket lock, batched calls claim slots by CAS and
+                                take it to grow a full chain */
 #define LSB_LOCK_FREE 1u     /* writers claim slots with CAS on slab words; growing a
                                 full chain takes the bucket lock */
 #define LSB_LOCK_RW 2u       /* reference-style: readers take a shared bucket lock too */

@@ -284,7 +284,8 @@ struct MapTraits {
   static constexpr bool kHasValue = true;
   // Without the bucket lock (LSB_LOCK_FREE) a dead slot may be reused only by
   // its own key: a reader that matched the old key could otherwise read the
-  // new key's value.  Locked inserts reuse any dead slot (scan_chain).
+  // new key's value.  The engine's inserts into other tables reuse any dead
+  // slot (table_insert_absent).
   static constexpr bool kReuseDead = false;
   __device__ static uint64_t hash(Key k) { return mix64(k); }
 };
@@ -585,10 +586,10 @@ __device__ __forceinline__ void table_find_n(const TableView& t, const typename 
 // Exactly one thread applies a given key at a time (the batch engine groups
 // same-key ops and lets only the group's last op write), so a key's slot is
 // only ever written by that thread.  Different keys of one bucket are kept
-// apart by the bucket lock (kLockWriter / kLockRW) or by CAS on the tag and
-// link words (kLockFree).  Order of writes for an insert: slot contents,
-// fence, tag byte (or link word): a lock-free reader that sees the live tag
-// sees the slot.
+// apart by CAS on the tag words; the bucket's lock word is taken to grow a full
+// chain.  LSB_LOCK_FREE tables (table_apply_lockfree) claim a slot with a busy
+// mark and set the live tag last, so that a reader that sees a live tag sees
+// the slot; the others (table_insert_absent) rely on the engine's phase order.
 template <class Tr>
 __device__ __forceinline__ void key_store(uint8_t* slot_ptr, typename Tr::Key key, uint64_t val) {
   if constexpr (Tr::kHasValue)
@@ -614,10 +615,8 @@ struct ScanResult {
   uint32_t tail;       // last slab of the chain
 };
 
-// kReuse: a dead slot of another key counts as free (the set always; the
-// map only under the bucket lock: a lock-free map reader that matched the
-// old key could otherwise read the new key's value, whereas the batch engine
-// never runs a reader while a locked writer runs).
+// kReuse: a dead slot of another key counts as free (the set; a lock-free map
+// reader that matched the old key could otherwise read the new key's value).
 template <class Tr, bool kReuse>
 __device__ __forceinline__ bool scan_chain(const TableView& t, typename Tr::Key key, uint64_t h,
                                            ScanResult& r, uint32_t start) {
@@ -674,48 +673,112 @@ __device__ __forceinline__ uint32_t* tag_word(uint8_t* slab, int slot) {
   return (uint32_t*)(slab + 4 + 4 * (slot >> 2));
 }
 
-// Under the bucket's writer lock.  The engine calls it while no kernel reads
-// the table, so only the lock's next holder looks at what it stores: the slot,
-// its tag and a new slab's link are plain stores in front of the releasing
-// unlock, with no fence of their own (a 2^18-op set batch's 105k inserts:
-// resolve 38 us with a fence before each tag and on both sides of the lock, 33
-// this way).
+// Slots a new key may take: empty ones and removed ones (nonzero, top bit clear).
+__device__ __forceinline__ uint32_t free_mask(const Meta& m) {
+  uint32_t fr = tag_match(m, 0u);
+#pragma unroll
+  for (int w = 0; w < 7; ++w) {
+    const uint32_t x = m.tag[w];
+    const uint32_t nz = ((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x;  // top bit set iff byte != 0
+    const uint32_t dead = nz & ~x & 0x80808080u;
+    uint32_t b = (dead >> 7) & 0x01010101u;
+    b = b | (b >> 7);
+    b = (b | (b >> 14)) & 0xFu;
+    fr |= b << (4 * w);
+  }
+  return fr & ((1u << kSlots) - 1u);
+}
+
+// Insert a key that the window's probe did not find (the engine's writes; one
+// thread per key, and no kernel reads the table meanwhile).  The slot is claimed
+// by a compare-and-swap of its tag word from the word that the scan saw to one
+// with the live tag, and then filled: nothing looks into a slot with a live tag
+// before the window ends, so the claim needs no lock, no busy mark and no
+// fence.  A removed slot of the same key is taken before any other (a key has
+// one slot at most); if another insert claims it first, this key simply has no
+// slot any more.  Tags change only from free to live and, for other keys'
+// slots, from live to removed, so a word that still compares equal is
+// unchanged.  The bucket's lock serves only to grow a full chain.
+// (Under the lock, an insert's chain was lock, tags, stores, releasing store,
+// and inserts into one bucket waited for one another: two 2^18-op set batches
+// with 131k inserts 116 us, 96 this way; 2^20 inserts into 2^16 empty buckets
+// 294 us a call, 207.)
 template <class Tr>
-__device__ void table_apply_locked(const TableView& t, typename Tr::Key key, uint64_t h,
-                                   bool present, uint64_t val) {
-  const uint32_t bucket = (uint32_t)h & t.mask;
-  if (!lock_writer(t, bucket)) return;
-  const uint32_t fp = fingerprint(h);
-  ScanResult r;
-  r.found_slot = -1;
-  r.free_slot = -1;
-  bool found = scan_chain<Tr, true>(t, key, h, r, bucket);
-  if (found) {
-    uint8_t* slab = slab_ptr(t.slabs, r.found_slab, Tr::kSlabBytes);
-    uint8_t* tagp = slab + 4 + r.found_slot;
-    if (present) {
-      if constexpr (Tr::kHasValue)
-        st_cg_u64(slab + kMetaBytes + r.found_slot * Tr::kSlotBytes + 8, val);
-      if (!r.found_live) st_cg_u8(tagp, (uint8_t)(0x80u | fp));
-    } else if (r.found_live) {
-      st_cg_u8(tagp, (uint8_t)fp);
+__device__ void table_insert_absent(const TableView& t, typename Tr::Key key, uint64_t h,
+                                    uint64_t val) {
+  const uint32_t bucket = (uint32_t)h & t.mask, fp = fingerprint(h);
+  uint32_t start = bucket;
+  for (uint32_t attempt = 0; attempt < kLockPolls; ++attempt) {
+    uint32_t s = start, at_slab = 0, at_word = 0;
+    int at = -1;       // the slot to claim, in slab at_slab; at_word = its tag word
+    bool own = false;  // it is the key's own removed slot
+    bool ended = false;
+    for (uint32_t hop = 0; hop < kMaxHops; ++hop) {
+      const uint8_t* slab = slab_ptr((const uint8_t*)t.slabs, s, Tr::kSlabBytes);
+      const Meta m = load_meta(slab);
+      for (uint32_t cand = tag_match(m, fp * 0x01010101u); cand && !own; cand &= cand - 1) {
+        const int slot = __ffs(cand) - 1;
+        if (key_load<Tr>(slab + kMetaBytes + slot * Tr::kSlotBytes) == key) {
+          own = true;
+          at = slot;
+          at_slab = s;
+        }
+      }
+      if (at < 0) {
+        uint32_t fr = free_mask(m);
+        // the first free slot (near the tags); after a lost race, another one
+        for (uint32_t skip = attempt ? (attempt + (uint32_t)(h >> 56)) % kSlots : 0u;
+             skip && (fr & (fr - 1u)); --skip)
+          fr &= fr - 1u;
+        if (fr) {
+          at = __ffs(fr) - 1;
+          at_slab = s;
+        }
+      }
+      if (at >= 0 && at_slab == s) {
+#pragma unroll
+        for (int w = 0; w < 7; ++w)
+          if (w == at >> 2) at_word = m.tag[w];
+      }
+      if (own || m.next == 0) {
+        ended = true;
+        break;
+      }
+      s = m.next;
     }
-  } else if (present) {
-    if (r.free_slot >= 0) {
-      uint8_t* slab = slab_ptr(t.slabs, r.free_slab, Tr::kSlabBytes);
-      key_store<Tr>(slab + kMetaBytes + r.free_slot * Tr::kSlotBytes, key, val);
-      st_cg_u8(slab + 4 + r.free_slot, (uint8_t)(0x80u | fp));
-    } else {
-      uint32_t n = pool_alloc(t);
+    if (!ended) {
+      raise_status(t.status, kStatusChain);
+      return;
+    }
+    if (at >= 0) {
+      uint8_t* slab = slab_ptr(t.slabs, at_slab, Tr::kSlabBytes);
+      const uint32_t sh = 8 * (at & 3);
+      const uint32_t claimed = (at_word & ~(0xFFu << sh)) | ((0x80u | fp) << sh);
+      if (atomicCAS(tag_word(slab, at), at_word, claimed) == at_word) {
+        key_store<Tr>(slab + kMetaBytes + at * Tr::kSlotBytes, key, val);
+        return;
+      }
+      start = bucket;
+      continue;
+    }
+    // the chain is full: grow it by one slab under the bucket's lock word
+    if (!lock_writer(t, bucket)) return;  // timeout raised
+    uint32_t* link = (uint32_t*)slab_ptr(t.slabs, s, Tr::kSlabBytes);
+    bool oom = false;
+    if (ld_cg_u32(link) == 0) {
+      const uint32_t n = pool_alloc(t);  // zeroed: every slot empty
       if (n != 0) {
-        uint8_t* slab = slab_ptr(t.slabs, n, Tr::kSlabBytes);
-        key_store<Tr>(slab + kMetaBytes, key, val);
-        st_cg_u8(slab + 4, (uint8_t)(0x80u | fp));
-        st_cg_u32(slab_ptr(t.slabs, r.tail, Tr::kSlabBytes), n);
+        __threadfence();
+        atomicExch(link, n);
+      } else {
+        oom = true;  // raised by pool_alloc
       }
     }
+    unlock_writer(t, bucket);
+    if (oom) return;
+    start = s;  // its successor now exists; the slabs before it hold no slot of the key
   }
-  unlock_writer(t, bucket);
+  raise_status(t.status, kStatusTimeout);
 }
 
 template <class Tr>
@@ -811,27 +874,22 @@ __device__ void table_apply_lockfree(const TableView& t, typename Tr::Key key, u
   raise_status(t.status, kStatusTimeout);
 }
 
-template <class Tr>
-__device__ __forceinline__ void table_apply(const TableView& t, typename Tr::Key key, uint64_t h,
-                                            bool present, uint64_t val) {
-  if (t.lock_mode == kLockFree)
-    table_apply_lockfree<Tr>(t, key, h, present, val);
-  else
-    table_apply_locked<Tr>(t, key, h, present, val);
-}
-
 // Write the final state of a key whose live slot is known from this window's
 // probe (loc has kLocLive).  Only this thread writes that key, and a live
 // slot keeps its key until its own key's writer tombstones it, so neither a
 // lock nor a rescan is needed: an update is one value store, a removal clears
 // the live bit of the tag with an atomic (other bytes of the word may be
-// changing under other writers).  Absent keys take table_apply.
+// changing under other writers).  Absent keys are inserted.
 template <class Tr>
 __device__ __forceinline__ void table_apply_known(const TableView& t, typename Tr::Key key,
                                                   uint64_t h, uint64_t loc, bool present,
                                                   uint64_t val) {
   if (!(loc & kLocLive)) {
-    if (present) table_apply<Tr>(t, key, h, true, val);
+    if (!present) return;
+    if (t.lock_mode == kLockFree)
+      table_apply_lockfree<Tr>(t, key, h, true, val);
+    else
+      table_insert_absent<Tr>(t, key, h, val);
     return;
   }
   // the location was read back from window scratch: check it before use
