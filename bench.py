@@ -543,9 +543,9 @@ def run_ours(args, world, rank, local):
     windows = args.steps * ((n + (1 << 20) - 1) >> 20)  # default window: 2^20 ops
     if overlap:
         form = ("batched call (execute_fused) over the queue of timed batches, one 2^20-op "
-                "window per batch: its reads in the lean read kernel on the caller's stream "
-                "while its puts are listed, probed, grouped and ordered on a second, "
-                "higher-priority stream, then one resolve launch (value); the same call one "
+                "window per batch: its ops are looked up in the lean read kernel on a second "
+                "stream while its puts are listed, grouped and ordered on the caller's, then "
+                "one resolve launch (value); the same call one "
                 "batch at a time (per_batch_launch_value); per-op-type calls: a get call and "
                 "a put call per batch (plain_value)")
         launches = 5 * windows
