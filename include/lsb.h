@@ -121,9 +121,9 @@ typedef struct lsb_tuning {
                              reading a slab's slots together); 0 = one op per thread,
                              tag sector then candidate slot (default, faster) */
   uint32_t overlap;       /* mixed batches (execute, execute_fused): 1 = each window runs
-                             as launches on two streams, the reads through the lean read
-                             kernel while the mutations are listed, probed, grouped and
-                             ordered on a higher-priority stream; the mutations are applied
+                             as launches on two streams, its ops looked up in the lean read
+                             kernel on the table's stream while the mutations are listed,
+                             grouped and ordered on the caller's; the mutations are applied
                              after both (read-mostly windows of many ops); 0 = per-phase
                              launches on the caller's stream (execute) and the persistent
                              kernel (execute_fused) */

@@ -26,6 +26,7 @@ constexpr uint32_t kMaxWindow = 1u << 23;  // owner field of a group slot is 24 
 constexpr uint32_t kTraceCap = 1024;        // phase-trace entries per fused launch
 constexpr uint32_t kFusedEpochs = kEpochs;  // odd epochs 1..253 for fused windows
 constexpr uint32_t kPlainEpochs = kEpochs;  // even epochs 2..254 for per-phase windows
+constexpr uint32_t kCapturedEpoch = 255;   // per-phase windows of a captured graph
 constexpr uint32_t kMaxFusedWindows = 16383;  // of one launch
 // One allocation for everything a fused launch zeroes first: two window
 // counter sets, the grid barrier, two region-counter sets.
@@ -1329,12 +1330,22 @@ struct Table {
 
   // Epoch of the next per-phase window (even: 2, 4, ...; the fused path uses
   // odd ones on the device); clears the group and chunk tables when they wrap.
+  // A window that is being captured runs again with every replay, between
+  // windows of any epoch: it clears the tables each time and takes an epoch
+  // that no other window uses.
   int next_plain_epoch(cudaStream_t s, uint32_t* e) {
-    if (epoch + 1 > kPlainEpochs) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    LSB_CK(cudaStreamIsCapturing(s, &cs));
+    const bool captured = cs == cudaStreamCaptureStatusActive;
+    if (captured || epoch + 1 > kPlainEpochs) {
       LSB_CK(cudaMemsetAsync(sc.gtab, 0, sizeof(uint64_t) * (sc.gmask + 1ull), s));
       LSB_CK(cudaMemsetAsync(sc.ctab, 0, sizeof(uint64_t) * (sc.cmask + 1ull), s));
-      epoch = 0;
     }
+    if (captured) {
+      *e = kCapturedEpoch;
+      return LSB_OK;
+    }
+    if (epoch + 1 > kPlainEpochs) epoch = 0;
     epoch += 1;
     *e = 2 * epoch;
     return LSB_OK;

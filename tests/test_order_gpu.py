@@ -69,3 +69,36 @@ def test_many_windows_of_one_call(cuda, fused):
         got, want = results(out), o.mixed(t, k, v)
         assert same_results(got, want), first_mismatch(got, want)
     assert m.status() == 0
+
+
+def test_captured_calls_replay_between_live_ones(cuda):
+    """put and remove calls captured into a caller's CUDA graph, replayed more
+    often than there are window epochs, with live calls on the same keys in
+    between: every result equals the oracle's."""
+    import torch
+    rng = np.random.default_rng(47)
+    n = 3000
+    k = W.key_of_rank(8, rng.integers(0, 200, size=n))  # groups of ~15: ordered lists
+    v, v2 = W.splitmix64(10, 0, n), W.splitmix64(11, 0, n)
+    m, o = Map(8), OracleMap(8)
+    dk, dv, dv2, part = dev(k), dev(v), dev(v2), dev(k[:500])
+    old = torch.zeros(n, dtype=torch.int64, device="cuda")
+    out = results_buf(500)
+    live = torch.zeros(n, dtype=torch.int64, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        m.put(dk, dv, old)
+        m.remove(part, out)
+    for r in range(140):
+        graph.replay()
+        m.put(dk, dv2, live)
+        want_old = o.put(k, v)
+        want_out = o.remove(k[:500])
+        want_live = o.put(k, v2)
+        if r % 10 == 9 or r < 3:
+            torch.cuda.synchronize()
+            assert np.array_equal(old.cpu().numpy().view(np.uint64), want_old), f"replay {r}"
+            got = results(out)
+            assert same_results(got, want_out), first_mismatch(got, want_out)
+            assert np.array_equal(live.cpu().numpy().view(np.uint64), want_live), f"replay {r}"
+    assert m.status() == 0
