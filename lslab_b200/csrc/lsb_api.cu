@@ -59,11 +59,6 @@ inline bool aligned(const void* p, size_t a) { return ((uintptr_t)p & (a - 1)) =
 #ifndef LSB_FUSED_LEAN_READS
 #define LSB_FUSED_LEAN_READS 1
 #endif
-// threads per block of the ordering kernel k_sort (one block per SM; a
-// block orders one big group at a time)
-#ifndef LSB_SORT_THREADS
-#define LSB_SORT_THREADS 256
-#endif
 // two read lookups in flight per thread in the fused kernel's lean read
 // loop: measured slower at the 64-register cap (more spills), so off
 #ifndef LSB_FUSED_READ_PAIR
@@ -1572,7 +1567,13 @@ struct Table {
   // room (2.4 us behind the probe; put of 52k keys 32.7 us with it, 29.4
   // without).
   int launch_sort(Window<Tr> w, cudaStream_t s, const uint32_t* dev_epoch) {
-    LSB_CK(launch_after(k_sort<Tr>, num_sms, LSB_SORT_THREADS, kSortSmemBytes, s,
+    // One block an SM, a big group at a time.  Twice the threads halve the
+    // passes over a group, which pays where groups are big, and cost 0.3 us
+    // where there is none (256 / 512, us a call: puts of Zipf keys 10k 19.0 /
+    // 18.9, 52k 29.0 / 26.5, 2^20 272 / 247; 80/15/5 window 172 / 166; six set
+    // calls without a big group 79.5 / 80.9).
+    const unsigned threads = w.n > 1u << 15 ? 512 : 256;
+    LSB_CK(launch_after(k_sort<Tr>, num_sms, threads, kSortSmemBytes, s,
                         w.n > kHugeSteps, sc, w, bar, dev_epoch));
     return LSB_OK;
   }
