@@ -148,15 +148,17 @@ __device__ __forceinline__ void store_read(void* out, uint32_t out_kind, uint32_
 }
 
 // Read-only batch (get / contains) in its lean form: one op per thread, no
-// grouping, no work claims, the result written straight out; with `types`,
-// the ops of a mixed window, whose mutations get their tentative result here
-// and their slot in mloc (their groups are formed elsewhere).  The code is
-// kept within 32 registers a thread (launch bound 256 x 8), so 2048 threads
+// grouping, no work claims, the result written straight out; with kMixed, the
+// ops of a mixed window, whose mutations get their tentative result here and
+// their slot in mloc (their groups are formed elsewhere).  Two kernels, since
+// in a table that L2 holds the instructions count (2^23 gets of 2^16 buckets
+// 124 us; 131 with the types' test in the one kernel).  The code is kept within
+// 32 registers a thread (launch bound 256 x 8), so 2048 threads
 // fit an SM: a lookup is two dependent loads (meta sector, then the
 // candidate slot), latency-bound, and twice the resident warps keep twice
 // the lookups in flight.  The first candidate is tried inline; a second
 // candidate or a longer chain continues in find_rest.
-template <class Tr>
+template <class Tr, bool kMixed>
 __global__ void __launch_bounds__(256, 8)
     k_read(TableView t, const uint8_t* types, const typename Tr::Key* keys, void* out,
            uint32_t out_kind, uint32_t n, uint64_t* mloc) {
@@ -164,17 +166,23 @@ __global__ void __launch_bounds__(256, 8)
   begin_after_previous();
   // one op per thread with a grid of n threads; a smaller grid strides
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint8_t type = types != nullptr ? __ldcs(types + i) : (uint8_t)kOpRead;
     Key key;
     if constexpr (sizeof(Key) == 8)
       key = (Key)ld_cs_u64(keys + i);
     else
       key = (Key)ld_cs_u32(keys + i);
-    uint64_t val, loc;
-    bool found = lean_lookup<Tr>(t, key, &val, &loc);
-    if (type != kOpRead) {
-      mloc[i] = loc;
-      if (out_kind == kOutBool) found |= type == kOpWrite;  // inserts report true
+    uint64_t val;
+    bool found;
+    if constexpr (kMixed) {
+      const uint8_t type = __ldcs(types + i);
+      uint64_t loc;
+      found = lean_lookup<Tr>(t, key, &val, &loc);
+      if (type != kOpRead) {
+        mloc[i] = loc;
+        if (out_kind == kOutBool) found |= type == kOpWrite;  // inserts report true
+      }
+    } else {
+      found = read_lookup<Tr>(t, key, &val);
     }
     store_read(out, out_kind, i, found, val);
   }
@@ -1440,7 +1448,7 @@ struct Table {
           k_read_coop<Tr><<<(m + 255) / 256, 256, 0, s>>>(view(), keys + off, o,
                                                           out ? out_kind : kOutNone, m);
         else
-          launch_after(k_read<Tr>, (m + 255) / 256, 256, 0, s, false, view(), nullptr, keys + off, o,
+          launch_after(k_read<Tr, false>, (m + 255) / 256, 256, 0, s, false, view(), nullptr, keys + off, o,
                        out ? out_kind : kOutNone, m, nullptr);
         LSB_CK(cudaGetLastError());
       }
@@ -1516,7 +1524,7 @@ struct Table {
         if (ordered_reads(m)) {
           if (int e2 = launch_read_ordered(w.types, w.keys, w.out, w.out_kind, m, side)) return e2;
         } else {
-          k_read<Tr><<<(m + 255) / 256, 256, 0, side>>>(view(), w.types, w.keys, w.out, w.out_kind,
+          k_read<Tr, true><<<(m + 255) / 256, 256, 0, side>>>(view(), w.types, w.keys, w.out, w.out_kind,
                                                         m, sc.mloc);
         }
         if (int e2 = span_mark(wi, 4, side)) return e2;
