@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(1024, 1)
   const uint32_t slot = fused_epoch != nullptr ? dev_window_slot(fused_epoch) : 0u;
   if (fused_epoch != nullptr) w.epoch = 2 * slot + 1;
   phase_resolve_mutations<Tr>(t, sc, w, tid, nt);
-  phase_resolve_reads<Tr>(sc, w, tid, nt);
+  phase_resolve_reads<Tr, true>(sc, w, tid, nt);
   release_counters(sc.cnt, bar, nullptr, 0, fused_epoch, slot + 1);
 }
 
@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(1024, 1)
   phase_sort_big<Tr>(sc, w, smem);
   __syncthreads();
   phase_resolve_mutations<Tr>(t, sc, w, threadIdx.x, blockDim.x);
-  phase_resolve_reads<Tr>(sc, w, threadIdx.x, blockDim.x);
+  phase_resolve_reads<Tr, true>(sc, w, threadIdx.x, blockDim.x);
   release_counters(sc.cnt, bar, nullptr, 0);
 }
 
@@ -651,10 +651,13 @@ __device__ void fused_windows(const TableView& t, const Scratch& sc, const Fused
         if (rt < ms)
           phase_resolve_mutations<Tr>(t, sc, w, rt, ms);
         else
-          phase_resolve_reads<Tr>(sc, w, rt - ms, rn - ms);
+          phase_resolve_reads<Tr, false>(sc, w, rt - ms, rn - ms);
       } else {
         phase_resolve_mutations<Tr>(t, sc, w, rt, rn);
-        phase_resolve_reads<Tr>(sc, w, rt, rn);
+        if (w.n > 1u << 20)
+          phase_resolve_reads<Tr, true>(sc, w, rt, rn);
+        else
+          phase_resolve_reads<Tr, false>(sc, w, rt, rn);
       }
     }
     // Before the next window: its probes must see this window's writes, and
