@@ -57,12 +57,19 @@ constexpr uint32_t kSortSmall = 4096;  // members a shared-memory sort holds
 constexpr uint32_t kHugeMin = 4096;
 constexpr uint32_t kHugeSteps = 1u << 17;
 constexpr uint32_t kRangeMembers = 1024;  // mean members of a range
+constexpr uint32_t kRangeTake = 3072;     // members aimed at when a range is cut again
+constexpr uint32_t kSampleMin = 16384;    // members from which the cuts follow from a sample
+constexpr uint32_t kSample = 256;         // members that the ranges' cuts follow from
+constexpr uint32_t kKnots = 32;           // pieces of the line through them
+constexpr uint32_t kSampleStep = kSample / kKnots;
 // the shared-memory sort: members rank themselves against all others up to
 // kRankAll, in a bitmap of the index range where that is at most
 // kBitWords * 32 wide, and by counting into kSortBins ranges otherwise
 constexpr uint32_t kRankAll = 256;
 constexpr uint32_t kBitWords = 2048;
+static_assert(kSample <= kRankAll, "the sample's sort leaves the chunk places alone");
 constexpr uint32_t kSortBins = 4096;  // index ranges of the shared-memory sort
+constexpr uint32_t kBinCrowd = 128;   // members of one of them that call for narrower ones
 // shared memory of the sort: members, members by range, range counts
 constexpr uint32_t kSortSmemBytes = (2 * kSortSmall + kSortBins + kSortBins / 32) * 4;
 // Word of range b: one word of padding per 32, so that threads scanning 4, 8
@@ -1035,8 +1042,10 @@ __device__ void block_lnu(const Scratch& sc, const Window<Tr>& w, const uint32_t
 //    itself against the few others of its range, so the cost follows the
 //    group's size and not the window's (a bitmap of the whole of a 2^20-op
 //    window took 16 passes: 118 us for the ordering of a window of the 80/15/5
-//    queue, 67 this way).  Ranges are at most 256 ops wide in such a window,
-//    which bounds the ranking for members packed into a few of them.
+//    queue, 67 this way).  Up to kSortBins / 4 members a quarter of the ranges
+//    does, unless many members share one, which makes the ranking long: then
+//    all of them, at most 256 ops wide in such a window (1,000 neighbours and
+//    one op far off: persistent form 99 us a call, 67 this way).
 __device__ inline const uint32_t* order_members(uint32_t n, uint32_t c, uint32_t lo, uint32_t hi,
                                                 uint32_t* mem, uint32_t* sorted,
                                                 uint32_t* bins) {
@@ -1088,16 +1097,21 @@ __device__ inline const uint32_t* order_members(uint32_t n, uint32_t c, uint32_t
     __syncthreads();
     return sorted;
   }
-  const uint32_t nb = c <= kSortBins / 4 ? kSortBins / 4 : kSortBins;
-  uint32_t sh = 0;
-  while (lo < hi && ((hi - lo) >> sh) >= nb) ++sh;
-  for (uint32_t k = tid; k < bin_word(nb); k += nt) bins[k] = 0;
-  __syncthreads();
-  for (uint32_t j = tid; j < c; j += nt) {
-    const uint32_t x = mem[j];
-    if (x < n) atomicAdd(&bins[bin_word((x - lo) >> sh)], 1u);
+  uint32_t nb = c <= kSortBins / 4 ? kSortBins / 4 : kSortBins, sh = 0;
+  for (;;) {
+    while (lo < hi && ((hi - lo) >> sh) >= nb) ++sh;
+    for (uint32_t k = tid; k < bin_word(nb); k += nt) bins[k] = 0;
+    __syncthreads();
+    bool crowded = false;
+    for (uint32_t j = tid; j < c; j += nt) {
+      const uint32_t x = mem[j];
+      if (x < n) crowded |= atomicAdd(&bins[bin_word((x - lo) >> sh)], 1u) >= kBinCrowd;
+    }
+    // few wide ranges and members packed into some of them: finer ones
+    if (!__syncthreads_or(crowded) || nb == kSortBins) break;
+    nb = kSortBins;
+    sh = 0;
   }
-  __syncthreads();
   const uint32_t per = (nb + nt - 1) / nt, b0 = tid * per;
   for (uint32_t k = b0; k < min(b0 + per, nb); ++k) local += bins[bin_word(k)];
   uint32_t run = block_exclusive_scan(local, s_tmp, &total);
@@ -1283,117 +1297,229 @@ __device__ __forceinline__ uint32_t huge_groups(const Scratch& sc, const WinCoun
   return min(ld_settled(&c->huge_count), sc.hcap);
 }
 
-// Members of group gslot (c of them) with lo <= index < hi, in any order, into
-// mem[0..kSortSmall); *cnt their number (it may exceed kSortSmall; the surplus
-// is not stored), *below the number of members under lo, *prev and *carry
-// 1 + the largest of those and 1 + the largest that is not an update (0 =
-// none; carry only with upd).  Whole block; the four are shared variables.
+// What gather_range finds out about a group beside the members it stores.
+struct RangeInfo {
+  uint32_t cnt;    // members with lo <= index < hi (may exceed kSortSmall; the surplus is not stored)
+  uint32_t below;  // members under lo
+  uint32_t prev;   // 1 + the largest of those (0 = none)
+  uint32_t carry;  // 1 + the largest of those that is not an update (0 = none; only with upd)
+  uint32_t rest;   // members with hi <= index < end
+  uint32_t next;   // the smallest of those
+};
+
+// Where the chunks of group gslot (c members) are, into places[]
+// (kHugeSteps / kChunk of them fit), so that loads of members depend on
+// nothing but shared memory.  Whole block; settled by the caller's barrier.
+__device__ inline void find_chunks(const Scratch& sc, uint32_t epoch, uint32_t gslot, uint32_t c,
+                                   uint32_t* places) {
+  const uint32_t nchunks = (c - kInline + kChunk - 1) / kChunk;
+  for (uint32_t k = threadIdx.x; k < nchunks; k += blockDim.x)
+    places[k] = chunk_find(sc, epoch, gslot, k);
+}
+
+// Members of group gslot (c of them, its chunks at places[]) with
+// lo <= index < hi, in any order, into mem[0..kSortSmall).  Whole block; *info
+// is a shared variable.  A block reads the whole group for each of its ranges,
+// so this is most of a hot key's ordering: a lane loads four members at a
+// time, twice before it looks at any, and a warp's members of the range are
+// counted together (ten keys of 100,000: 340 us with a word a lane and a count
+// each, 253 with two loads, 245 with four; but four unroll to twice the code,
+// which a short group's few steps wait for: ordering of a window of the
+// 80/15/5 queue 20.8 us, 20.9 and 22.5).
 template <class Tr>
 __device__ void gather_range(const Scratch& sc, const Window<Tr>& w, uint32_t gslot, uint32_t c,
-                             uint32_t lo, uint32_t hi, bool upd, uint32_t* mem,
-                             uint32_t* places, uint32_t* cnt, uint32_t* below, uint32_t* prev,
-                             uint32_t* carry) {
-  constexpr uint32_t kUnits = 8;  // chunks a warp reads at a time
+                             uint32_t lo, uint32_t hi, uint32_t end, bool upd, uint32_t* mem,
+                             const uint32_t* places, RangeInfo* info) {
+  constexpr uint32_t kLoads = 2, kQuads = kChunk / 4, kStep = kLoads * 32 / kQuads;
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-  // every chunk's place first (kHugeSteps / kChunk of them fit `places`), so
-  // that the chunk loads depend on nothing but shared memory
-  const uint32_t nchunks = (c - kInline + kChunk - 1) / kChunk;
-  for (uint32_t k = tid; k < nchunks; k += blockDim.x)
-    places[k] = chunk_find(sc, w.epoch, gslot, k);
-  if (tid == 0) *cnt = *below = *prev = *carry = 0;
+  if (tid == 0) {
+    info->cnt = info->below = info->prev = info->carry = info->rest = 0;
+    info->next = 0xFFFFFFFFu;
+  }
   __syncthreads();
-  uint32_t my_below = 0, my_prev = 0, my_carry = 0;
-  auto take = [&](uint32_t x) {  // whole warp
-    const bool in = x < w.n && x >= lo && x < hi;
-    const uint32_t m = __ballot_sync(0xFFFFFFFFu, in);
-    if (m) {
-      uint32_t at = 0;
-      if (lane == (uint32_t)__ffs(m) - 1) at = atomicAdd(cnt, (uint32_t)__popc(m));
-      at = __shfl_sync(0xFFFFFFFFu, at, __ffs(m) - 1) + __popc(m & ((1u << lane) - 1u));
-      if (in && at < kSortSmall) mem[at] = x;
+  uint32_t my_below = 0, my_prev = 0, my_carry = 0, my_rest = 0, my_next = 0xFFFFFFFFu;
+  // a lane's members (0xFFFFFFFF: none); whole warp
+  auto take = [&](const auto& x) {
+    uint32_t in = 0;
+#pragma unroll
+    for (uint32_t e = 0; e < sizeof(x) / 4; ++e) {
+      const uint32_t v = x[e];
+      if (v < lo) {
+        ++my_below;
+        my_prev = max(my_prev, v + 1);
+        if (upd && v + 1 > my_carry && op_type(w, v) != kOpUpdate) my_carry = v + 1;
+      } else if (v < hi) {
+        ++in;
+      } else {
+        my_rest += v < end;
+        my_next = min(my_next, v);
+      }
     }
-    if (x < lo) {
-      ++my_below;
-      my_prev = max(my_prev, x + 1);
-      if (upd && x + 1 > my_carry && op_type(w, x) != kOpUpdate) my_carry = x + 1;
+    if (!__ballot_sync(0xFFFFFFFFu, in != 0)) return;
+    uint32_t upto = in;  // of the lanes up to this one
+#pragma unroll
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, upto, d);
+      if (lane >= d) upto += y;
     }
+    uint32_t at = 0;
+    if (lane == 31) at = atomicAdd(&info->cnt, upto);
+    at = __shfl_sync(0xFFFFFFFFu, at, 31) + upto - in;
+#pragma unroll
+    for (uint32_t e = 0; e < sizeof(x) / 4; ++e)
+      if (x[e] >= lo && x[e] < hi) {
+        if (at < kSortSmall) mem[at] = x[e];
+        ++at;
+      }
   };
-  if (warp == 0)
-    take(lane < kInline ? ld_cg_u32(&sc.ginl[(size_t)gslot * kInline + lane]) : 0xFFFFFFFFu);
-  for (uint32_t k0 = warp * kUnits; k0 < nchunks; k0 += nwarps * kUnits) {
-    uint32_t x[kUnits];
+  const uint32_t whole = (c - kInline) / kChunk;  // chunks without a hole
+  if (warp == 0) {  // the inline members and the last chunk's
+    const uint32_t j = kInline + whole * kChunk + lane;
+    const uint32_t s = j < c ? places[whole] : 0xFFFFFFFFu;
+    const uint32_t x[2] = {
+        lane < kInline ? ld_cg_u32(&sc.ginl[(size_t)gslot * kInline + lane]) : 0xFFFFFFFFu,
+        s != 0xFFFFFFFFu ? ld_cg_u32(&sc.cdat[(size_t)s * kChunk + lane]) : 0xFFFFFFFFu};
+    take(x);
+  }
+  for (uint32_t k0 = warp * kStep; k0 < whole; k0 += nwarps * kStep) {
+    uint32_t x[4 * kLoads];
 #pragma unroll
-    for (uint32_t q = 0; q < kUnits; ++q) {
-      const uint32_t s = k0 + q < nchunks ? places[k0 + q] : 0xFFFFFFFFu;
-      const uint32_t j = kInline + (k0 + q) * kChunk + lane;
-      x[q] = (j < c && s != 0xFFFFFFFFu) ? ld_cg_u32(&sc.cdat[(size_t)s * kChunk + lane])
-                                         : 0xFFFFFFFFu;
+    for (uint32_t q = 0; q < kLoads; ++q) {
+      const uint32_t k = k0 + q * (32 / kQuads) + lane / kQuads;
+      const uint32_t s = k < whole ? places[k] : 0xFFFFFFFFu;
+      uint4 v = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu};
+      if (s != 0xFFFFFFFFu) v = ld_cg_v4(&sc.cdat[(size_t)s * kChunk + 4 * (lane % kQuads)]);
+      x[4 * q] = v.x;
+      x[4 * q + 1] = v.y;
+      x[4 * q + 2] = v.z;
+      x[4 * q + 3] = v.w;
     }
-#pragma unroll
-    for (uint32_t q = 0; q < kUnits; ++q) take(x[q]);
+    take(x);
   }
   my_below = __reduce_add_sync(0xFFFFFFFFu, my_below);
   my_prev = __reduce_max_sync(0xFFFFFFFFu, my_prev);
   my_carry = __reduce_max_sync(0xFFFFFFFFu, my_carry);
+  my_rest = __reduce_add_sync(0xFFFFFFFFu, my_rest);
+  my_next = __reduce_min_sync(0xFFFFFFFFu, my_next);
   if (lane == 0) {
-    atomicAdd(below, my_below);
-    atomicMax(prev, my_prev);
-    atomicMax(carry, my_carry);
+    atomicAdd(&info->below, my_below);
+    atomicMax(&info->prev, my_prev);
+    atomicMax(&info->carry, my_carry);
+    atomicAdd(&info->rest, my_rest);
+    atomicMin(&info->next, my_next);
   }
   __syncthreads();
 }
 
-// Members of group gslot (c of them) with lo <= index < end, ordered by the
-// whole block: their part of the group's list at seg[off ..) and their
+// Where to cut [lo, end) so that about kRangeTake of its m members come first,
+// if they lie evenly: the least width always fits the shared-memory sort.
+__device__ __forceinline__ uint32_t range_cut(uint32_t lo, uint32_t end, uint32_t m) {
+  if (m <= kSortSmall || end - lo <= kSortSmall) return end;
+  return lo + max(kSortSmall, (uint32_t)((uint64_t)(end - lo) * kRangeTake / m));
+}
+
+// Range r of `ranges` of group gslot (c members), ordered by the whole block:
+// its part of the group's list, which begins at seg[off], and its members'
 // predecessors.
+//
+// Without `sampled` the ranges are equal pieces of the window from `first` on.
+// With it, kSample members at even steps of the group's storage are ordered,
+// every kSampleStep-th of them is a knot, and the ranges are equal pieces of
+// the line through the knots: they hold about as many members each wherever
+// these lie in the window (a burst, a batch in key order), and every block
+// finds the same cuts for itself.  The sample is two more round trips (3 us of
+// a block), which a short group's few reads do not earn.  Where a range holds
+// more members than fit the sort, it is cut again by their number, and
+// stretches without a member are skipped.  (Cut into steps of kSortSmall
+// indices instead, and never by a sample, one block read the group twice for
+// each of them: mixed call of 2^20 ops with 5,000 puts of one key in a row at
+// its end 420 us, now 68; 20,000 284, now 72; 130,000 244, now 97; an even
+// spread of 100,000 155, now 155.  With four grid steps for all groups above
+// kHugeMin: 117, 127, 127 and 184.)
 template <class Tr>
 __device__ void sort_range(const Scratch& sc, const Window<Tr>& w, uint32_t gslot, uint32_t c,
-                           uint32_t off, uint32_t lo, uint32_t end, bool upd, uint32_t* smem) {
-  __shared__ uint32_t s_cnt, s_below, s_prev, s_carry;
-  uint32_t* sorted = smem + kSortSmall;
+                           uint32_t off, uint32_t first, uint32_t r, uint32_t ranges,
+                           bool sampled, bool upd, uint32_t* smem) {
+  __shared__ RangeInfo s_info;
+  uint32_t *sorted = smem + kSortSmall, *places = sorted + kSortSmall;
+  find_chunks(sc, w.epoch, gslot, c, places);
+  __syncthreads();
+  const uint32_t* list = sorted;
+  if (sampled) {
+    for (uint32_t q = threadIdx.x; q < kSample; q += blockDim.x) {
+      const uint32_t j = (uint32_t)((uint64_t)q * c / kSample);
+      const uint32_t s = j < kInline ? 0u : places[(j - kInline) / kChunk];
+      const uint32_t* p = j < kInline ? &sc.ginl[(size_t)gslot * kInline + j]
+                                      : &sc.cdat[(size_t)s * kChunk + (j - kInline) % kChunk];
+      smem[q] = s == 0xFFFFFFFFu ? s : ld_cg_u32(p);
+    }
+    __syncthreads();
+    list = order_members(w.n, kSample, 1, 0, smem, sorted, places);
+  }
+  auto cut = [&](uint32_t k) -> uint32_t {  // the least index of range k
+    if (k == 0) return 0;
+    if (k >= ranges) return w.n;
+    if (!sampled) return first + (uint32_t)((uint64_t)(w.n - first) * k / ranges);
+    const uint32_t at = k * kKnots, q = at / ranges;
+    const uint32_t a = list[q * kSampleStep];
+    const uint32_t b = list[min((q + 1) * kSampleStep, kSample - 1)];
+    if (a >= w.n || b >= w.n) return w.n;  // (holes sort last)
+    return a + (b - a) * (at % ranges) / ranges;
+  };
+  uint32_t lo = cut(r);
+  const uint32_t end = cut(r + 1);
   uint32_t hi = end;
-  while (lo < end) {
-    gather_range<Tr>(sc, w, gslot, c, lo, hi, upd, smem, sorted + kSortSmall, &s_cnt, &s_below,
-                     &s_prev, &s_carry);
-    const uint32_t cnt = s_cnt, below = s_below, prev = s_prev, carry = s_carry;
-    if (cnt > kSortSmall) {  // members crowd here: as many indices as surely fit
-      hi = lo + kSortSmall;
-      __syncthreads();  // the counts are cleared again
+  bool found = true;  // places[] holds the chunks (the sort of a sample needs no bins)
+  while (lo < end) {  // block-uniform
+    if (!found) find_chunks(sc, w.epoch, gslot, c, places);
+    found = true;
+    gather_range<Tr>(sc, w, gslot, c, lo, hi, end, upd, smem, places, &s_info);
+    const RangeInfo i = s_info;
+    if (i.cnt > kSortSmall && hi - lo > kSortSmall) {
+      hi = range_cut(lo, hi, i.cnt);
+      __syncthreads();  // s_info is cleared again
       continue;
     }
-    const uint32_t* list = order_members(w.n, cnt, lo, hi - 1, smem, sorted, sorted + kSortSmall);
+    const uint32_t cnt = min(i.cnt, kSortSmall);
+    list = order_members(w.n, cnt, lo, hi - 1, smem, sorted, places);
+    found = false;
     for (uint32_t j = threadIdx.x; j < cnt; j += blockDim.x) {
-      const uint32_t x = list[j], p = j ? list[j - 1] + 1 : prev;
-      if (x < w.n && below + j < c) {
-        sc.seg[off + below + j] = x;
-        sc.pred[x] = p | (below + j + 1 == c ? kPredLast : 0u);
+      const uint32_t x = list[j], p = j ? list[j - 1] + 1 : i.prev;
+      if (x < w.n && i.below + j < c) {
+        sc.seg[off + i.below + j] = x;
+        sc.pred[x] = p | (i.below + j + 1 == c ? kPredLast : 0u);
       }
     }
     __syncthreads();
-    if (upd) block_lnu<Tr>(sc, w, list, cnt, carry);
-    lo = hi;
-    hi = end;
+    if (upd) block_lnu<Tr>(sc, w, list, cnt, i.carry);
+    if (i.rest == 0) break;
+    lo = i.next;
+    hi = range_cut(lo, end, i.rest);
   }
 }
 
-// Groups of kHugeMin+1 .. kHugeSteps members (hot keys).  The window's indices
-// from its first mutation on are cut into equal ranges of about kRangeMembers
-// members, one job each; a block reads the whole group for its range, so it
-// knows the range's place in the group's list and the member before it, and no
-// block waits for another.  Reading the group once per range is cheap while it
-// is at most half a MB in L2, and it replaces four grid steps with barriers
-// between them (ordering of a window of the 80/15/5 queue 67 -> 39 us).  Jobs go to blocks by a static stride that starts behind
-// the blocks with a group of their own.  The lists fill seg from its end (other
-// groups from its start: all lists together hold at most max_window members).
+// Groups of kHugeMin+1 .. kHugeSteps members (hot keys), cut into ranges of
+// about kRangeMembers members, one job each (sort_range); a block reads the
+// whole group for its range, so it knows the range's place in the group's list
+// and the member before it, and no block waits for another.  Reading the group
+// once per range is cheap while it is at most half a MB in L2, and it replaces
+// four grid steps with barriers between them (ordering of a window of the
+// 80/15/5 queue 67 -> 39 us).  Jobs go to blocks by a static stride that starts
+// behind the blocks with a group of their own.  The lists fill seg from its end
+// (other groups from its start: all lists together hold at most max_window
+// members).  With more ranges than blocks they are twice as long and cut by a
+// sample, since every range costs a read of its group (2^20 puts in key order:
+// ten keys of 100,000 291 us with 1024 members a range, 235 with 2048; 209 keys
+// of 5,000 371 us in equal pieces, 230 by samples; grid steps 267 and 740).
 template <class Tr>
 __device__ void sort_ranges(const Scratch& sc, const Window<Tr>& w, uint32_t* smem, uint32_t job0,
                             bool upd) {
   const uint32_t lane = threadIdx.x & 31, g = gridDim.x;
   // no mutation lies before it (0 when it was not recorded)
-  const uint32_t inv = ld_settled(&w.cnt->inv_first_mut), first = inv ? ~inv : 0u;
+  const uint32_t inv = ld_settled(&w.cnt->inv_first_mut), first = inv ? min(~inv, w.n) : 0u;
   const uint32_t H = huge_groups(sc, w.cnt);
-  if (first >= w.n) return;
   uint32_t job = job0 % g, used = 0;  // jobs and seg entries of the groups before
+  bool crowded = H > 32;
   for (uint32_t h0 = 0; h0 < H; h0 += 32) {
     uint32_t gs = 0, cs = 0;  // lane l: group h0 + l
     if (h0 + lane < H) {
@@ -1401,6 +1527,8 @@ __device__ void sort_ranges(const Scratch& sc, const Window<Tr>& w, uint32_t* sm
       cs = min(g_count(ld_relaxed_u64(&sc.gtab[gs])), w.n);
       if (cs > kHugeSteps || cs <= kHugeMin) cs = 0;
     }
+    crowded |= __reduce_add_sync(0xFFFFFFFFu, cs) / kRangeMembers > g;
+    const uint32_t share = crowded ? 2 * kRangeMembers : kRangeMembers;
     for (uint32_t q = 0; q < 32; ++q) {
       const uint32_t c = __shfl_sync(0xFFFFFFFFu, cs, q);
       const uint32_t gslot = __shfl_sync(0xFFFFFFFFu, gs, q);
@@ -1408,12 +1536,10 @@ __device__ void sort_ranges(const Scratch& sc, const Window<Tr>& w, uint32_t* sm
       used += c;
       if (used > sc.max_window) return;  // cannot happen: members are distinct ops
       const uint32_t off = sc.max_window - used;
-      const uint32_t ranges = (c + kRangeMembers - 1) / kRangeMembers;
-      const uint32_t width = (w.n - first + ranges - 1) / ranges;
+      const uint32_t ranges = (c + share - 1) / share;
       for (uint32_t r = (blockIdx.x + g - job) % g; r < ranges; r += g) {
         if (r == 0 && threadIdx.x == 0) sc.goff[gslot] = off;
-        sort_range<Tr>(sc, w, gslot, c, off, first + r * width, min(w.n, first + (r + 1) * width),
-                       upd, smem);
+        sort_range<Tr>(sc, w, gslot, c, off, first, r, ranges, crowded || c > kSampleMin, upd, smem);
       }
       job = (job + ranges) % g;
     }
