@@ -26,7 +26,6 @@ constexpr uint32_t kMaxWindow = 1u << 23;  // owner field of a group slot is 24 
 constexpr uint32_t kTraceCap = 1024;        // phase-trace entries per fused launch
 constexpr uint32_t kFusedEpochs = kEpochs;  // odd epochs 1..253 for fused windows
 constexpr uint32_t kPlainEpochs = kEpochs;  // even epochs 2..254 for per-phase windows
-constexpr uint32_t kCapturedEpoch = 255;   // per-phase windows of a captured graph
 constexpr uint32_t kMaxFusedWindows = 16383;  // of one launch
 // One allocation for everything a fused launch zeroes first: two window
 // counter sets, the grid barrier, two region-counter sets.
@@ -98,10 +97,42 @@ inline cudaError_t launch_after(void (*f)(P...), unsigned grid, unsigned block, 
   return cudaLaunchKernelEx(&cfg, f, static_cast<P>(a)...);
 }
 
+// Windows run as launches on two streams (Table::run_plain, tuning overlap)
+// and per-phase windows that are being captured take their epochs from the
+// device counter of the fused path, so a CUDA graph of them can be replayed:
+// every kernel of the window reads the counter f (written only by the window's
+// last block, in k_resolve or k_finish) and uses epoch 2f+1, or 1 after the
+// tables were cleared when the epochs ran out.
+__device__ __forceinline__ uint32_t dev_window_slot(const uint32_t* fused_epoch) {
+  const uint32_t f = ld_cg_u32(fused_epoch);
+  return f + 1 > kFusedEpochs ? 0u : f;
+}
+
+// The group tables are cleared by the grid when the device epochs ran out, in
+// the first kernel of a window that takes one (its joins follow in the next).
+__device__ __forceinline__ void clear_spent_tables(const Scratch& sc, const uint32_t* fused_epoch) {
+  if (ld_cg_u32(fused_epoch) + 1 <= kFusedEpochs) return;
+  const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t nt = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = tid; i <= sc.gmask; i += nt) sc.gtab[i] = 0;
+  for (size_t i = tid; i <= sc.cmask; i += nt) sc.ctab[i] = 0;
+}
+
+// First kernel of a captured per-phase window.  (Two memsets of both tables in
+// front of each such window need no counter, but cost as much as the call:
+// puts captured one behind the other, 500 keys each 17.2 us and 12.7 this way,
+// 20,000 keys 23.0 and 17.7.)
+__global__ void __launch_bounds__(256) k_open_window(Scratch sc, const uint32_t* fused_epoch) {
+  begin_after_previous();
+  clear_spent_tables(sc, fused_epoch);
+}
+
 template <class Tr, bool kGroup, int P>
 __global__ void __launch_bounds__(1024, LSB_PROBE_MIN_BLOCKS)
-    k_probe(TableView t, Scratch sc, Window<Tr> w, uint32_t chunk, uint32_t dedup) {
+    k_probe(TableView t, Scratch sc, Window<Tr> w, uint32_t chunk, uint32_t dedup,
+            const uint32_t* fused_epoch) {
   begin_after_previous();
+  if (kGroup && fused_epoch != nullptr) w.epoch = 2 * dev_window_slot(fused_epoch) + 1;
   const uint32_t warp = spread_warp();
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   phase_probe<Tr, kGroup, P>(t, sc, w, warp, nwarps, &w.cnt->probe_cursor, chunk, dedup != 0);
@@ -109,28 +140,22 @@ __global__ void __launch_bounds__(1024, LSB_PROBE_MIN_BLOCKS)
 
 // Phase A of a per-phase window of at most one round of lookups: the first
 // join_blocks blocks join the mutations to their groups, the others look all
-// ops up.
-template <class Tr>
+// ops up.  kCaptured: the window takes its epoch from *fused_epoch (a test of
+// the pointer at run time cost puts of 777 keys 0.35 of 10.2 us).
+template <class Tr, bool kCaptured>
 __global__ void __launch_bounds__(256, 6)
-    k_lookup_join(TableView t, Scratch sc, Window<Tr> w, uint32_t join_blocks) {
+    k_lookup_join(TableView t, Scratch sc, Window<Tr> w, uint32_t join_blocks,
+                  const uint32_t* fused_epoch) {
   __shared__ uint8_t slices[8][kJoinSpan];
   begin_after_previous();
   const uint32_t warp = threadIdx.x >> 5;
-  if (blockIdx.x < join_blocks)
+  if (blockIdx.x < join_blocks) {
+    if constexpr (kCaptured) w.epoch = 2 * dev_window_slot(fused_epoch) + 1;
     phase_join<Tr>(sc, w, warp * join_blocks + blockIdx.x, join_blocks * 8, slices[warp]);
-  else
+  } else {
     phase_lookup<Tr>(t, sc, w, (blockIdx.x - join_blocks) * 256 + threadIdx.x,
                      (gridDim.x - join_blocks) * 256);
-}
-
-// Windows run as launches on two streams (Table::run_plain, tuning overlap)
-// take their epochs from the device counter of the fused path, so a CUDA
-// graph of them can be replayed: every kernel of the window reads the
-// counter f (written only by the window's last block, in k_resolve) and uses
-// epoch 2f+1, or 1 after the tables were cleared when the epochs ran out.
-__device__ __forceinline__ uint32_t dev_window_slot(const uint32_t* fused_epoch) {
-  const uint32_t f = ld_cg_u32(fused_epoch);
-  return f + 1 > kFusedEpochs ? 0u : f;
+  }
 }
 
 // A read's result in the caller's layout.
@@ -410,12 +435,7 @@ template <class Tr>
 __global__ void __launch_bounds__(256) k_list_muts(Scratch sc, Window<Tr> w,
                                                    const uint32_t* fused_epoch) {
   begin_after_previous();
-  if (ld_cg_u32(fused_epoch) + 1 > kFusedEpochs) {  // epochs ran out: clear the tables
-    const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t nt = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = tid; i <= sc.gmask; i += nt) sc.gtab[i] = 0;
-    for (size_t i = tid; i <= sc.cmask; i += nt) sc.ctab[i] = 0;
-  }
+  clear_spent_tables(sc, fused_epoch);
   phase_list_muts<Tr>(sc, w, spread_warp(), (gridDim.x * blockDim.x) >> 5);
 }
 
@@ -458,16 +478,21 @@ __global__ void __launch_bounds__(1024, 1)
 // kernels; 512: 15.2 and 15.9).
 constexpr uint32_t kFinishOps = 512;
 
-template <class Tr>
+template <class Tr, bool kCaptured>
 __global__ void __launch_bounds__(1024, 1)
-    k_finish(TableView t, Scratch sc, Window<Tr> w, GridBarrier* bar) {
+    k_finish(TableView t, Scratch sc, Window<Tr> w, GridBarrier* bar, uint32_t* fused_epoch) {
   extern __shared__ __align__(16) uint32_t smem[];
   begin_after_previous();
+  uint32_t slot = 0;
+  if constexpr (kCaptured) {
+    slot = dev_window_slot(fused_epoch);
+    w.epoch = 2 * slot + 1;
+  }
   phase_sort_big<Tr>(sc, w, smem);
   __syncthreads();
   phase_resolve_mutations<Tr>(t, sc, w, threadIdx.x, blockDim.x);
   phase_resolve_reads<Tr, true>(sc, w, threadIdx.x, blockDim.x);
-  release_counters(sc.cnt, bar, nullptr, 0);
+  release_counters(sc.cnt, bar, nullptr, 0, kCaptured ? fused_epoch : nullptr, slot + 1);
 }
 
 // One batch split into windows, all phases of all windows in one cooperative
@@ -1292,7 +1317,9 @@ struct Table {
     bins = reinterpret_cast<BinCounters*>(reinterpret_cast<uint8_t*>(sc.cnt) + kBinsOffset);
     LSB_CK(cudaFuncSetAttribute(k_sort<Tr>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kSortSmemBytes));
-    LSB_CK(cudaFuncSetAttribute(k_finish<Tr>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    LSB_CK(cudaFuncSetAttribute((k_finish<Tr, false>), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kSortSmemBytes));
+    LSB_CK(cudaFuncSetAttribute((k_finish<Tr, true>), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kSortSmemBytes));
     LSB_CK(cudaFuncSetAttribute(k_fused<Tr, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kSortSmemBytes));
@@ -1336,22 +1363,12 @@ struct Table {
 
   // Epoch of the next per-phase window (even: 2, 4, ...; the fused path uses
   // odd ones on the device); clears the group and chunk tables when they wrap.
-  // A window that is being captured runs again with every replay, between
-  // windows of any epoch: it clears the tables each time and takes an epoch
-  // that no other window uses.
   int next_plain_epoch(cudaStream_t s, uint32_t* e) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    LSB_CK(cudaStreamIsCapturing(s, &cs));
-    const bool captured = cs == cudaStreamCaptureStatusActive;
-    if (captured || epoch + 1 > kPlainEpochs) {
+    if (epoch + 1 > kPlainEpochs) {
       LSB_CK(cudaMemsetAsync(sc.gtab, 0, sizeof(uint64_t) * (sc.gmask + 1ull), s));
       LSB_CK(cudaMemsetAsync(sc.ctab, 0, sizeof(uint64_t) * (sc.cmask + 1ull), s));
+      epoch = 0;
     }
-    if (captured) {
-      *e = kCapturedEpoch;
-      return LSB_OK;
-    }
-    if (epoch + 1 > kPlainEpochs) epoch = 0;
     epoch += 1;
     *e = 2 * epoch;
     return LSB_OK;
@@ -1385,10 +1402,11 @@ struct Table {
   }
 
   template <bool kGroup>
-  void launch_probe(int grid, const Window<Tr>& w, cudaStream_t s) {
+  void launch_probe(int grid, const Window<Tr>& w, cudaStream_t s,
+                    const uint32_t* dev_epoch = nullptr) {
     auto* f = tune.prefetch == 0 ? k_probe<Tr, kGroup, 1>
             : tune.prefetch == 1 ? k_probe<Tr, kGroup, 2> : k_probe<Tr, kGroup, 3>;
-    launch_after(f, grid, tune.block, 0, s, false, view(), sc, w, tune.chunk, tune.dedup);
+    launch_after(f, grid, tune.block, 0, s, false, view(), sc, w, tune.chunk, tune.dedup, dev_epoch);
   }
 
   // Whether a window of m ops is probed as lookups beside joins
@@ -1403,10 +1421,11 @@ struct Table {
            lock_mode != kLockRW;
   }
 
-  void launch_lookup_join(const Window<Tr>& w, cudaStream_t s) {
+  void launch_lookup_join(const Window<Tr>& w, cudaStream_t s, const uint32_t* dev_epoch) {
     const uint32_t look = (w.n + 255) / 256;
     const uint32_t join = std::min<uint32_t>(look, num_sms * 2);
-    launch_after(k_lookup_join<Tr>, look + join, 256, 0, s, false, view(), sc, w, join);
+    launch_after(dev_epoch ? k_lookup_join<Tr, true> : k_lookup_join<Tr, false>, look + join, 256,
+                 0, s, false, view(), sc, w, join, dev_epoch);
   }
 
   // Read-only batch: the lean read kernel (k_read), or, with in-warp dedup
@@ -1490,14 +1509,19 @@ struct Table {
       const bool overlap = types != nullptr && tune.overlap && !tune.dedup &&
                            lock_mode != kLockRW && kstride == 1 && out_kind != kOutOld &&
                            out_kind != kOutOld32;
-      if (!overlap) {
+      // a window that is being captured runs again with every replay, between
+      // windows of any kind: it takes its epoch on the device too
+      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+      if (!overlap) LSB_CK(cudaStreamIsCapturing(s, &cs));
+      const bool captured = cs == cudaStreamCaptureStatusActive;
+      if (!overlap && !captured) {
         int e = next_plain_epoch(s, &w.epoch);
         if (e) return e;
       }
       w.cnt = &sc.cnt[0];
       // the counters and the sort launch's grid barrier are zero here: the
       // previous launch's last block cleared them (release_counters)
-      uint32_t* dev_epoch = overlap ? fused_epoch : nullptr;
+      uint32_t* dev_epoch = overlap || captured ? fused_epoch : nullptr;
       const int wi = (int)(off / W);
       if (overlap && off == 0) span_windows = 0;
       if (overlap) {
@@ -1534,16 +1558,18 @@ struct Table {
         LSB_CK(cudaEventRecord(ev_join, side));
         LSB_CK(cudaStreamWaitEvent(s, ev_join, 0));
       } else {
+        if (captured) launch_after(k_open_window, num_sms, 256, 0, s, false, sc, fused_epoch);
         if (split_probe(m))
-          launch_lookup_join(w, s);
+          launch_lookup_join(w, s, dev_epoch);
         else
-          launch_probe<true>(grid_for(m), w, s);
+          launch_probe<true>(grid_for(m), w, s, dev_epoch);
         if (m <= kFinishOps) {
-          launch_after(k_finish<Tr>, 1, 1024, kSortSmemBytes, s, false, view(), sc, w, bar);
+          launch_after(captured ? k_finish<Tr, true> : k_finish<Tr, false>, 1, 1024, kSortSmemBytes,
+                       s, false, view(), sc, w, bar, dev_epoch);
           LSB_CK(cudaGetLastError());
           continue;
         }
-        if (int e2 = launch_sort(w, s, nullptr)) return e2;
+        if (int e2 = launch_sort(w, s, dev_epoch)) return e2;
       }
       // One wave of blocks at most: the step's work is the window's
       // mutations (and the reads after its first one), walked by a grid

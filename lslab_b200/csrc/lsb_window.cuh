@@ -196,7 +196,7 @@ struct Window {
   uint32_t kstride;      // elements between consecutive keys (2 for AoS pairs)
   uint32_t vstride;      // elements between consecutive values
   uint32_t n;
-  uint32_t epoch;        // 1..255
+  uint32_t epoch;        // 1..254: odd from the device's counter, even from the host's
   uint8_t uniform;
   uint8_t out_kind;
   uint8_t v32;           // values are 32-bit (stored zero-extended)
