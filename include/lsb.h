@@ -495,7 +495,12 @@ int lsb_kvs_remove(lsb_kvs* s, const uint64_t* keys, uint8_t* found_out, size_t 
 int lsb_kvs_usage(lsb_kvs* s, uint64_t* heap_used, uint64_t* heap_dead, uint64_t* heap_cap,
                   cudaStream_t stream);
 /* Move the live values to the front of the heap (key order) and drop the
- * garbage; must not overlap other calls on the store.  Synchronises. */
+ * garbage; must not overlap other calls on the store.  Synchronises.  Entries
+ * that a caller wrote into the map itself (lsb_kvs_map) count too: two keys
+ * with one handle become two values.  LSB_ERR_STATE (no effect) when such a
+ * handle reaches past the heap or the live values no longer fit it;
+ * LSB_ERR_OOM (no effect) without room for the scratch: the live bytes and 32
+ * bytes an entry, of which a store keeps up to 64 MB for the next call. */
 int lsb_kvs_compact(lsb_kvs* s, cudaStream_t stream);
 
 /* ---- device per-warp API -------------------------------------------------

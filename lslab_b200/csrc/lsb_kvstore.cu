@@ -43,6 +43,7 @@ struct HostWords {
   uint64_t first, last;  // put: the batch's first and last offset
   uint64_t total;        // get, compact: bytes of all found (live) values
   uint64_t count;        // compact: live entries
+  uint64_t end;          // compact: the largest end of a live value in the heap
   uint32_t bad;          // put: a value longer than kMaxLen or offsets that fall
   uint32_t pad;
 };
@@ -84,6 +85,7 @@ __global__ void k_dead_bytes(const lsb_result* res, const uint64_t* old, uint32_
 // 1024 consecutive items twice, took 151 us for 32768 lengths; the two launches
 // take 7.)
 constexpr uint32_t kParts = 1024;
+constexpr uint32_t kSums = 5;  // words behind the parts, of k_live
 constexpr uint32_t kPartThreads = 256;
 
 inline uint32_t part_size(uint64_t n) {  // a multiple of the block, at least 4 tiles
@@ -230,16 +232,17 @@ __global__ void __launch_bounds__(256)
 
 // ------------------------------------------------------- heap compaction
 // The live entries of a table as (key, address of the slot's value): a warp
-// per bucket, a lane per slot.  With keys == nullptr only counts them and
-// their values' bytes into *words (through sums[0..1], cleared by the caller,
-// of which sums[2] blocks are done).
+// per bucket, a lane per slot.  With keys == nullptr only counts them, their
+// values' bytes and where the last of these ends into *words (through
+// sums[0..1] and sums[4], cleared by the caller, of which sums[2] blocks are
+// done).
 __global__ void __launch_bounds__(256)
     k_live(lsb::TableView t, uint32_t buckets, uint64_t* keys, uint64_t** slots, uint64_t cap,
            unsigned long long* sums, HostWords* words) {
   using Tr = lsb::MapTraits;
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  uint64_t count = 0, bytes = 0;
+  uint64_t count = 0, bytes = 0, end = 0;
   for (uint64_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < buckets; b += nw) {
     uint32_t s = (uint32_t)b;
     for (uint32_t hop = 0; hop < lsb::kMaxHops; ++hop) {
@@ -250,8 +253,10 @@ __global__ void __launch_bounds__(256)
       const uint8_t* sp = slab + lsb::kMetaBytes + lane * Tr::kSlotBytes;
       if (keys == nullptr) {
         if (mine) {
+          const uint64_t h = lsb::ld_cg_u64(sp + 8);
           ++count;
-          bytes += h_len(lsb::ld_cg_u64(sp + 8));
+          bytes += h_len(h);
+          end = max(end, h_off(h) + h_len(h));
         }
       } else if (live) {
         unsigned long long at = 0;
@@ -268,6 +273,8 @@ __global__ void __launch_bounds__(256)
   }
   if (keys != nullptr) return;
   __shared__ int last;
+  for (int d = 16; d > 0; d >>= 1) end = max(end, __shfl_xor_sync(0xFFFFFFFFu, end, d));
+  if (lane == 0 && end) atomicMax(&sums[4], (unsigned long long)end);
   count = block_sum(count);
   bytes = block_sum(bytes);
   if (threadIdx.x == 0) {
@@ -279,6 +286,7 @@ __global__ void __launch_bounds__(256)
       __threadfence();
       words->count = atomicAdd(&sums[0], 0ull);
       words->total = atomicAdd(&sums[1], 0ull);
+      words->end = atomicMax(&sums[4], 0ull);
     }
   }
 }
@@ -497,7 +505,7 @@ int lsb_kvs_create(unsigned log2_buckets, uint64_t heap_bytes, const lsb_options
   if (rc == LSB_OK &&
       (cudaMalloc(&s->heap, (heap_bytes + 3) / 4 * 4) != cudaSuccess ||  // whole words
        cudaMalloc(&s->dead, sizeof(unsigned long long)) != cudaSuccess ||
-       cudaMalloc(&s->parts, sizeof(uint64_t) * (kParts + 4)) != cudaSuccess ||
+       cudaMalloc(&s->parts, sizeof(uint64_t) * (kParts + kSums)) != cudaSuccess ||
        cudaHostAlloc((void**)&s->words, sizeof(HostWords), cudaHostAllocMapped) != cudaSuccess ||
        cudaHostGetDevicePointer((void**)&s->d_words, s->words, 0) != cudaSuccess ||
        cudaMemset(s->dead, 0, sizeof(unsigned long long)) != cudaSuccess)) {
@@ -637,12 +645,15 @@ int lsb_kvs_compact(lsb_kvs* s, cudaStream_t stream) {
   lsb_internal_map_view(s->map, &view, &buckets);
   unsigned long long* sums = reinterpret_cast<unsigned long long*>(s->parts + kParts);
   const uint32_t scan_blocks = (uint32_t)std::min<uint64_t>(((uint64_t)buckets + 7) / 8, 148 * 8);
-  if (cudaMemsetAsync(sums, 0, 4 * sizeof(*sums), stream) != cudaSuccess) return LSB_ERR_CUDA;
+  if (cudaMemsetAsync(sums, 0, kSums * sizeof(*sums), stream) != cudaSuccess) return LSB_ERR_CUDA;
   k_live<<<scan_blocks, 256, 0, stream>>>(view, buckets, nullptr, nullptr, 0, sums, s->d_words);
   if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(stream) != cudaSuccess)
     return LSB_ERR_CUDA;
   const uint64_t n = s->words->count, live = s->words->total;
-  if (live > s->heap_used) return LSB_ERR_STATE;  // the map holds handles that are not the store's
+  // The map may hold more entries than the store put (lsb_kvs_map): a handle
+  // under a second key is a value of its own from here on.  Refused: handles
+  // that reach past the heap, and more bytes than it takes.
+  if (s->words->end > s->heap_cap || live > s->heap_cap) return LSB_ERR_STATE;
   int rc = LSB_OK;
   if (n) {
     const uint32_t part = sort_part(n), blocks = (uint32_t)((n + part - 1) / part);
