@@ -55,7 +55,10 @@ constexpr uint32_t kSortSmall = 4096;  // members a shared-memory sort holds
 // members by several, each taking an index range (sort_ranges), and groups of
 // more than kHugeSteps by the huge_* steps between grid barriers
 constexpr uint32_t kHugeMin = 4096;
-constexpr uint32_t kHugeSteps = 1u << 17;
+#ifndef LSB_HUGE_STEPS  // (a build for tests takes the steps for smaller groups)
+#define LSB_HUGE_STEPS (1u << 17)
+#endif
+constexpr uint32_t kHugeSteps = LSB_HUGE_STEPS;
 constexpr uint32_t kRangeMembers = 1024;  // mean members of a range
 constexpr uint32_t kRangeTake = 3072;     // members aimed at when a range is cut again
 constexpr uint32_t kSampleMin = 16384;    // members from which the cuts follow from a sample
@@ -1748,7 +1751,7 @@ __device__ void huge_scatter(const Scratch& sc, const Window<Tr>& w, uint32_t gw
   for (uint32_t h = 0; h < H; ++h) {
     uint32_t gslot;
     const uint32_t c = huge_size(sc, w, h, &gslot);
-    if (c <= kHugeSteps) continue;  // sort_group_ranges ordered it
+    if (c <= kHugeSteps) continue;  // sort_ranges ordered it
     const uint32_t units = 1 + (c - kInline + kChunk - 1) / kChunk;
     uint32_t* bins = sc.hbins + (size_t)h * kHugeBins;
     const uint32_t* hrun = sc.hrun + (size_t)h * kHugeBins;
