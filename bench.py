@@ -941,9 +941,8 @@ def run_batches(args, world, rank, local):
         f_ms.append(e[0].elapsed_time(e[1]))
         p_ms.append(e[2].elapsed_time(e[3]))
         # the same per-op-type calls captured into one CUDA graph, so the GPU
-        # runs them without host issue gaps (captured afresh for each replay:
-        # a replay runs every captured window once, so no window epoch
-        # repeats).  The plain table takes the stream once more; a key's final
+        # runs them without host issue gaps (captured afresh for each
+        # repetition).  The plain table takes the stream once more; a key's final
         # state is its last mutation in the stream, so the contents still
         # equal the fused table's; results go to separate buffers.
         pg = torch.cuda.CUDAGraph()
@@ -1284,9 +1283,10 @@ def run_probes(args, world, rank, local):
 
 
 def run_locks(args, world, rank, local):
-    """Bucket-lock comparison on the map (writer lock = the reference's
-    warp_mutex role; lock-free = CAS on slab tag words; rw = reader-writer
-    locks on the read path too): 2^20-op batches, Zipf 0.99 over 2^26 keys on
+    """Bucket-lock comparison on the map (writer = inserts claim a slot by CAS,
+    any dead one too, and take the bucket's lock, the reference's warp_mutex, to
+    grow a chain; free = a claim with a busy mark, readers may run beside it;
+    rw = as writer, and readers take a shared lock): 2^20-op batches, Zipf 0.99 over 2^26 keys on
     2^22 buckets prefilled with 2^26 keys, 95/5 and 50/50 get/put, fused and
     per-op-type forms.  Results are identical across modes (tests)."""
     import torch

@@ -228,8 +228,8 @@ int lsb_map_set_tuning(lsb_map* m, const lsb_tuning* t);
  * windows (tuning overlap), the entries come from timing events instead, ns
  * counted from the first window's start, for each window (< 16, window field
  * = window & 31): phase 0 start, 1 read kernel done, 2 mutation steps
- * (listing, probing, ordering) done, 3 resolve done, and with window field
- * | 32: phase 1 listing done, phase 2 probing done.  Calls issued while the
+ * (listing, grouping, ordering) done, 3 resolve done, and with window field
+ * | 32: phase 1 listing done, phase 2 grouping done.  Calls issued while the
  * stream is being captured record none. */
 int lsb_map_set_trace(lsb_map* m, int on);
 int lsb_map_read_trace(lsb_map* m, uint64_t* out, size_t cap, size_t* count,

@@ -73,7 +73,10 @@ inline bool aligned(const void* p, size_t a) { return ((uintptr_t)p & (a - 1)) =
 // reads or writes any memory; a kernel launched in the usual way waits for
 // nothing here.  The next kernel is let in only after the wait: let in before
 // it, the kernels behind it start too, one behind the other, and hold room that
-// the running one needs (the six calls: 153 us).
+// the running one needs (the six calls: 153 us).  A cooperative launch may be a
+// dependent too: it starts when every block of the kernel before it has got
+// here, and so is resident and waits for nobody behind it, and its own blocks
+// get room as those end.
 __device__ __forceinline__ void begin_after_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
@@ -1175,8 +1178,8 @@ struct Table {
   bool binned = false;         // fused path probes in table-region order (measured slower)
   int fused_per_sm[3][4] = {};  // occupancy by (prefetch, block size) once queried
   int resolve_per_sm = 0;       // resident 256-thread k_resolve blocks per SM once queried
-  // tuning overlap: the lookups of a window run on `side` (lowest stream
-  // priority: the mutation steps on the caller's stream are the longer chain)
+  // tuning overlap: the lookups of a window run on `side`, a stream of default
+  // priority, which is the lowest there is
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   uint32_t* rhist = nullptr;  // region counts of ordered reads (+ the read count)
@@ -1317,19 +1320,15 @@ struct Table {
     bins = reinterpret_cast<BinCounters*>(reinterpret_cast<uint8_t*>(sc.cnt) + kBinsOffset);
     LSB_CK(cudaFuncSetAttribute(k_sort<Tr>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kSortSmemBytes));
-    LSB_CK(cudaFuncSetAttribute((k_finish<Tr, false>), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kSortSmemBytes));
-    LSB_CK(cudaFuncSetAttribute((k_finish<Tr, true>), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                kSortSmemBytes));
+    for (auto* f : {k_finish<Tr, false>, k_finish<Tr, true>})
+      LSB_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kSortSmemBytes));
     LSB_CK(cudaFuncSetAttribute(k_fused<Tr, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kSortSmemBytes));
     LSB_CK(cudaFuncSetAttribute(k_fused<Tr, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kSortSmemBytes));
     LSB_CK(cudaFuncSetAttribute(k_fused<Tr, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kSortSmemBytes));
-    int least = 0, greatest = 0;
-    LSB_CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-    LSB_CK(cudaStreamCreateWithPriority(&side, cudaStreamNonBlocking, least));
+    LSB_CK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
     LSB_CK(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
     LSB_CK(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
     return LSB_OK;
@@ -1406,7 +1405,8 @@ struct Table {
                     const uint32_t* dev_epoch = nullptr) {
     auto* f = tune.prefetch == 0 ? k_probe<Tr, kGroup, 1>
             : tune.prefetch == 1 ? k_probe<Tr, kGroup, 2> : k_probe<Tr, kGroup, 3>;
-    launch_after(f, grid, tune.block, 0, s, false, view(), sc, w, tune.chunk, tune.dedup, dev_epoch);
+    launch_after(f, grid, tune.block, 0, s, false, view(), sc, w, tune.chunk, tune.dedup,
+                 dev_epoch);
   }
 
   // Whether a window of m ops is probed as lookups beside joins

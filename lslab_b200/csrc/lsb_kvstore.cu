@@ -644,7 +644,12 @@ int lsb_kvs_compact(lsb_kvs* s, cudaStream_t stream) {
   uint32_t buckets = 0;
   lsb_internal_map_view(s->map, &view, &buckets);
   unsigned long long* sums = reinterpret_cast<unsigned long long*>(s->parts + kParts);
-  const uint32_t scan_blocks = (uint32_t)std::min<uint64_t>(((uint64_t)buckets + 7) / 8, 148 * 8);
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount,
+                             lsb_internal_map_device(s->map)) != cudaSuccess)
+    return LSB_ERR_CUDA;
+  const uint32_t scan_blocks =
+      (uint32_t)std::min<uint64_t>(((uint64_t)buckets + 7) / 8, (uint64_t)sms * 8);
   if (cudaMemsetAsync(sums, 0, kSums * sizeof(*sums), stream) != cudaSuccess) return LSB_ERR_CUDA;
   k_live<<<scan_blocks, 256, 0, stream>>>(view, buckets, nullptr, nullptr, 0, sums, s->d_words);
   if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(stream) != cudaSuccess)

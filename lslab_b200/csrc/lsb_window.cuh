@@ -7,18 +7,19 @@
 //   A probe    every op reads the table (pre-window state, P lookups in flight
 //              per thread) and writes that as its tentative result.  Each
 //              mutation joins its key's group in a scratch hash table
-//              (epoch-tagged slots, never cleared) and gets a position in it;
+//              (epoch-tagged slots, cleared when the epochs run out) and gets
+//              a position in it;
 //              positions 0..7 are stored inline in the group, later ones in
 //              32-entry chunks found through a second small hash table.  The
 //              mutation also records where its key lives (the probe's slot).
-//   D sort     only groups with more than 8 mutations: one block gathers the
-//              group, orders it by op index, stores the sorted list and every
-//              member's predecessor.  Skipped when no such group exists.
+//   D sort     only groups with more than 8 mutations: a warp, a block or, for
+//              hot keys, several blocks gather the group, order it by op index,
+//              store the sorted list and every member's predecessor.
 //   E resolve  a mutation takes its result from its predecessor in index
 //              order (that op's post-state: put -> {1, value}, remove ->
 //              {0, 0}); the group's last mutation writes the final state (a
-//              value store or tag flip at the recorded slot, or a locked
-//              insert for a key that was absent).  A read after the window's
+//              value store or tag flip at the recorded slot, or an insert for
+//              a key that was absent).  A read after the window's
 //              first mutation finds its key's group and, if a mutation of that
 //              key precedes it, takes that mutation's post-state.
 // Only phase E writes the table and only one thread per key does, so no probe
@@ -364,7 +365,8 @@ __device__ __forceinline__ void group_place(const Scratch& sc, const Window<Tr>&
   }
 }
 
-// The same, with the slot that the probe found for the op.
+// The same, with the slot that the probe found for the op (for joins one op at
+// a time).
 template <class Tr>
 __device__ __forceinline__ void group_store(const Scratch& sc, const Window<Tr>& w, uint32_t slot,
                                             uint32_t pos, uint32_t i, uint64_t loc) {
@@ -725,8 +727,10 @@ __device__ __forceinline__ void warp_sync() {
 // Joins: warp warp_id of num_warps takes spans of 32 ops.  When every warp has
 // one of 128 ops, it takes those instead and first packs their mutations, so
 // that the joins of a read-mostly mix run with full warps (and more same-key
-// ops share one); with fewer the packing would only leave warps idle.  `slice`
-// is kJoinSpan bytes of shared memory of the warp's own.
+// ops share one); with fewer the packing would only leave warps idle.  (The
+// launches of today have more warps than that for every window that is split,
+// so they take spans of 32.)  `slice` is kJoinSpan bytes of shared memory of
+// the warp's own.
 constexpr uint32_t kJoinSpan = 128;
 
 template <class Tr>
@@ -1219,9 +1223,10 @@ __device__ void sort_group_block(const Scratch& sc, const Window<Tr>& w, uint32_
 // before it and its last non-update predecessor a max-scan.  15 exchange
 // steps for 32 members and 21 for 64, against 32 K^2 compares a lane for
 // ranking each against all others (8 a lane, for groups of up to 256, measured
-// slower than a block each: 6 us for the one warp's 36 steps).  seg's space is taken with one atomic whose answer is first needed
-// for the stores.  The exchange loops stay rolled: the code runs once or twice a
-// launch, and unrolled its instruction fetches cost more than they save.
+// slower than a block each: 6 us for the one warp's 36 steps).  seg's space is
+// taken with one atomic whose answer is first needed for the stores.  The
+// exchange loops stay rolled: the code runs once or twice a launch, and
+// unrolled its instruction fetches cost more than they save.
 template <class Tr, int K>
 __device__ __forceinline__ void sort_group_warp(const Scratch& sc, const Window<Tr>& w,
                                              uint32_t gslot, uint32_t c, bool upd) {
@@ -1302,7 +1307,7 @@ __device__ __forceinline__ uint32_t huge_groups(const Scratch& sc, const WinCoun
 
 // What gather_range finds out about a group beside the members it stores.
 struct RangeInfo {
-  uint32_t cnt;    // members with lo <= index < hi (may exceed kSortSmall; the surplus is not stored)
+  uint32_t cnt;    // members with lo <= index < hi (those past kSortSmall are not stored)
   uint32_t below;  // members under lo
   uint32_t prev;   // 1 + the largest of those (0 = none)
   uint32_t carry;  // 1 + the largest of those that is not an update (0 = none; only with upd)
@@ -1542,7 +1547,8 @@ __device__ void sort_ranges(const Scratch& sc, const Window<Tr>& w, uint32_t* sm
       const uint32_t ranges = (c + share - 1) / share;
       for (uint32_t r = (blockIdx.x + g - job) % g; r < ranges; r += g) {
         if (r == 0 && threadIdx.x == 0) sc.goff[gslot] = off;
-        sort_range<Tr>(sc, w, gslot, c, off, first, r, ranges, crowded || c > kSampleMin, upd, smem);
+        sort_range<Tr>(sc, w, gslot, c, off, first, r, ranges, crowded || c > kSampleMin, upd,
+                       smem);
       }
       job = (job + ranges) % g;
     }
