@@ -138,7 +138,8 @@ typedef struct lsb_tuning {
                                 take it to grow a full chain */
 #define LSB_LOCK_FREE 1u     /* writers claim slots with CAS on slab words; growing a
                                 full chain takes the bucket lock */
-#define LSB_LOCK_RW 2u       /* reference-style: readers take a shared bucket lock too */
+#define LSB_LOCK_RW 2u       /* as LSB_LOCK_WRITER, and readers take a shared bucket lock
+                                (reference-style) */
 
 /* ---- map<uint64_t, uint64_t> ------------------------------------------
  * Replaces lslab::map<K,V>::map(unsigned n_log_2) (include/lslab/map.h:43-52)
