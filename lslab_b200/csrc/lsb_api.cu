@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(256)
 }
 
 // Ordering of the window's big groups; when hot keys produced groups of
-// more than kHugeSteps members, the grid (a cooperative launch) continues
+// more than steps_limit members, the grid (a cooperative launch) continues
 // with the huge_* steps between grid barriers.
 // fused_epoch: the window's epoch is the device one (the two-stream form).
 template <class Tr>
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(1024, 1)
   begin_after_previous();
   if (fused_epoch != nullptr) w.epoch = 2 * dev_window_slot(fused_epoch) + 1;
   phase_sort_big<Tr>(sc, w, smem);
-  if (ld_settled(&w.cnt->steps_count) == 0) return;  // grid-uniform: the probe kernel has ended
+  if (!takes_steps(w)) return;  // grid-uniform: the probe kernel has ended
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
   uint32_t seq = 0;
   huge_hist<Tr>(sc, w, gtid >> 5, gthreads >> 5);
@@ -638,7 +638,7 @@ __device__ void fused_windows(const TableView& t, const Scratch& sc, const Fused
     // skips below are grid-uniform
     const bool has_big = ld_settled(&w.cnt->big_count) != 0;
     const bool has_mut = ld_settled(&w.cnt->inv_first_mut) != 0;
-    const bool has_huge = ld_settled(&w.cnt->steps_count) != 0;
+    const bool has_huge = takes_steps(w);
     if (has_big || split < w.n) {
       if (has_big) phase_sort_big<Tr>(sc, w, smem);
       if (has_huge) huge_hist<Tr>(sc, w, warp, nwarps);
@@ -1599,7 +1599,7 @@ struct Table {
   }
 
   // Ordering of the window's big groups (k_sort).  A window of more than
-  // kHugeSteps ops may hold a group that takes its steps with grid barriers,
+  // kHugeSteps ops may hold groups that take the steps with grid barriers,
   // so it is a cooperative launch, which waits for all of its blocks to have
   // room (2.4 us behind the probe; put of 52k keys 32.7 us with it, 29.4
   // without).

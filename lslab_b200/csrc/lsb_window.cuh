@@ -54,18 +54,20 @@ constexpr uint32_t kWarpSort = 64;    // groups up to this size are ordered by o
 constexpr uint32_t kSortSmall = 4096;  // members a shared-memory sort holds
 // larger groups are ordered by one block each, groups of more than kHugeMin
 // members by several, each taking an index range (sort_ranges), and groups of
-// more than kHugeSteps by the huge_* steps between grid barriers
+// more than kHugeSteps by the huge_* steps between grid barriers (steps_limit)
 constexpr uint32_t kHugeMin = 4096;
 #ifndef LSB_HUGE_STEPS  // (a build for tests takes the steps for smaller groups)
 #define LSB_HUGE_STEPS (1u << 17)
 #endif
 constexpr uint32_t kHugeSteps = LSB_HUGE_STEPS;
+// with more than kHugeFew groups above kHugeMid those take the steps too
+constexpr uint32_t kHugeMid = kHugeSteps < 98304 ? kHugeSteps : 98304;
+constexpr uint32_t kHugeFew = 2;
 constexpr uint32_t kRangeMembers = 1024;  // mean members of a range
 constexpr uint32_t kRangeTake = 3072;     // members aimed at when a range is cut again
 constexpr uint32_t kSampleMin = 16384;    // members from which the cuts follow from a sample
 constexpr uint32_t kSample = 256;         // members that the ranges' cuts follow from
-constexpr uint32_t kKnots = 32;           // pieces of the line through them
-constexpr uint32_t kSampleStep = kSample / kKnots;
+constexpr uint32_t kSampleStep = 8;       // every eighth is a knot, every sixteenth for long ranges
 // the shared-memory sort: members rank themselves against all others up to
 // kRankAll, in a bitmap of the index range where that is at most
 // kBitWords * 32 wide, and by counting into kSortBins ranges otherwise
@@ -119,7 +121,8 @@ struct WinCounters {
   uint32_t run_count;      // runs of huge groups (each sorted by one block)
   uint32_t upd_count;      // updates among the window's mutations
   uint32_t steps_count;    // groups with more than kHugeSteps members
-  uint32_t pad[4];
+  uint32_t mid_count;      // groups with more than kHugeMid members
+  uint32_t pad[3];
   uint32_t mut_seg[kMutSegs * kSegStride];  // mutations listed per index range
 };
 
@@ -137,6 +140,7 @@ __device__ inline void win_counters_reset(WinCounters* c) {
   c->run_count = 0;
   c->upd_count = 0;
   c->steps_count = 0;
+  c->mid_count = 0;
 }
 
 // Scratch owned by a table, sized for max_window ops.
@@ -361,6 +365,7 @@ __device__ __forceinline__ void group_place(const Scratch& sc, const Window<Tr>&
       const uint32_t h = atomicAdd(&w.cnt->huge_count, 1u);
       if (h < sc.hcap) sc.hlist[h] = slot;
     }
+    if (pos == kHugeMid) atomicAdd(&w.cnt->mid_count, 1u);
     if (pos == kHugeSteps) atomicAdd(&w.cnt->steps_count, 1u);
   }
 }
@@ -1305,6 +1310,25 @@ __device__ __forceinline__ uint32_t huge_groups(const Scratch& sc, const WinCoun
   return min(ld_settled(&c->huge_count), sc.hcap);
 }
 
+// Members above which a group takes the grid steps.  A few hot keys are faster
+// by ranges, whose blocks wait for nobody (one key of 100,000 spread over 2^20
+// ops: 155 us a call, by steps 184), but the ranges read a group once each and
+// the steps a handful of times, which pays as soon as the ranges are more than
+// one round of blocks (mixed call of 2^20 ops, per-phase: two keys of 130,000
+// 181 us by ranges and 212 by steps, three 259 and 236; three of 70,000 160 and
+// 181; ten of 105,000 415 and 327; a window of 3 * 2^20 puts over thirty keys
+// 882 and 690, over eighty 586 and 747).
+template <class Tr>
+__device__ __forceinline__ uint32_t steps_limit(const Window<Tr>& w) {
+  return ld_settled(&w.cnt->mid_count) > kHugeFew ? kHugeMid : kHugeSteps;
+}
+
+// Whether a window has such a group (the same in every block).
+template <class Tr>
+__device__ __forceinline__ bool takes_steps(const Window<Tr>& w) {
+  return ld_settled(&w.cnt->steps_count) != 0 || ld_settled(&w.cnt->mid_count) > kHugeFew;
+}
+
 // What gather_range finds out about a group beside the members it stores.
 struct RangeInfo {
   uint32_t cnt;    // members with lo <= index < hi (those past kSortSmall are not stored)
@@ -1430,30 +1454,33 @@ __device__ __forceinline__ uint32_t range_cut(uint32_t lo, uint32_t end, uint32_
 // its part of the group's list, which begins at seg[off], and its members'
 // predecessors.
 //
-// Without `sampled` the ranges are equal pieces of the window from `first` on.
-// With it, kSample members at even steps of the group's storage are ordered,
-// every kSampleStep-th of them is a knot, and the ranges are equal pieces of
-// the line through the knots: they hold about as many members each wherever
-// these lie in the window (a burst, a batch in key order), and every block
-// finds the same cuts for itself.  The sample is two more round trips (3 us of
-// a block), which a short group's few reads do not earn.  Where a range holds
-// more members than fit the sort, it is cut again by their number, and
-// stretches without a member are skipped.  (Cut into steps of kSortSmall
-// indices instead, and never by a sample, one block read the group twice for
-// each of them: mixed call of 2^20 ops with 5,000 puts of one key in a row at
-// its end 420 us, now 68; 20,000 284, now 72; 130,000 244, now 97; an even
-// spread of 100,000 155, now 155.  With four grid steps for all groups above
-// kHugeMin: 117, 127, 127 and 184.)
+// With step 0 the ranges are equal pieces of the window from `first` on.
+// Otherwise kSample members at even steps of the group's storage are ordered,
+// every step-th of them is a knot, and the ranges are equal pieces of the line
+// through the knots: they hold about as many members each wherever these lie
+// in the window (a burst, a batch in key order), and every block finds the same
+// cuts for itself.  The fewer samples between two knots, the closer the line and
+// the less even the ranges; long ranges (half of what the sort takes, on
+// average) need them even (two keys of 130,000: 177 us a call, and 238 where one
+// of 32 pieces came out too long; 512 samples cost 2 to 8 us a call).  The
+// sample is two more round trips (3 us of a block), which a short group's few
+// reads do not earn.  Where a range holds more members than fit the sort, it is
+// cut again by their number, and stretches without a member are skipped.  (Cut
+// into steps of kSortSmall indices instead, and never by a sample, one block
+// read the group twice for each of them: mixed call of 2^20 ops with 5,000 puts
+// of one key in a row at its end 420 us, now 68; 20,000 284, now 71; 130,000
+// 244, now 101; an even spread of 100,000 155, now 158.  With four grid steps
+// for all groups above kHugeMin: 117, 127, 127 and 184.)
 template <class Tr>
 __device__ void sort_range(const Scratch& sc, const Window<Tr>& w, uint32_t gslot, uint32_t c,
                            uint32_t off, uint32_t first, uint32_t r, uint32_t ranges,
-                           bool sampled, bool upd, uint32_t* smem) {
+                           uint32_t step, bool upd, uint32_t* smem) {
   __shared__ RangeInfo s_info;
   uint32_t *sorted = smem + kSortSmall, *places = sorted + kSortSmall;
   find_chunks(sc, w.epoch, gslot, c, places);
   __syncthreads();
   const uint32_t* list = sorted;
-  if (sampled) {
+  if (step) {
     for (uint32_t q = threadIdx.x; q < kSample; q += blockDim.x) {
       const uint32_t j = (uint32_t)((uint64_t)q * c / kSample);
       const uint32_t s = j < kInline ? 0u : places[(j - kInline) / kChunk];
@@ -1467,10 +1494,9 @@ __device__ void sort_range(const Scratch& sc, const Window<Tr>& w, uint32_t gslo
   auto cut = [&](uint32_t k) -> uint32_t {  // the least index of range k
     if (k == 0) return 0;
     if (k >= ranges) return w.n;
-    if (!sampled) return first + (uint32_t)((uint64_t)(w.n - first) * k / ranges);
-    const uint32_t at = k * kKnots, q = at / ranges;
-    const uint32_t a = list[q * kSampleStep];
-    const uint32_t b = list[min((q + 1) * kSampleStep, kSample - 1)];
+    if (!step) return first + (uint32_t)((uint64_t)(w.n - first) * k / ranges);
+    const uint32_t at = k * (kSample / step), q = at / ranges;
+    const uint32_t a = list[q * step], b = list[min((q + 1) * step, kSample - 1)];
     if (a >= w.n || b >= w.n) return w.n;  // (holes sort last)
     return a + (b - a) * (at % ranges) / ranges;
   };
@@ -1506,7 +1532,7 @@ __device__ void sort_range(const Scratch& sc, const Window<Tr>& w, uint32_t gslo
   }
 }
 
-// Groups of kHugeMin+1 .. kHugeSteps members (hot keys), cut into ranges of
+// Groups of kHugeMin+1 .. steps_limit members (hot keys), cut into ranges of
 // about kRangeMembers members, one job each (sort_range); a block reads the
 // whole group for its range, so it knows the range's place in the group's list
 // and the member before it, and no block waits for another.  Reading the group
@@ -1517,15 +1543,15 @@ __device__ void sort_range(const Scratch& sc, const Window<Tr>& w, uint32_t gslo
 // (other groups from its start: all lists together hold at most max_window
 // members).  With more ranges than blocks they are twice as long and cut by a
 // sample, since every range costs a read of its group (2^20 puts in key order:
-// ten keys of 100,000 291 us with 1024 members a range, 235 with 2048; 209 keys
-// of 5,000 371 us in equal pieces, 230 by samples; grid steps 267 and 740).
+// 52 keys of 20,000 198 us with 1024 members a range, 160 with 2048; 209 keys
+// of 5,000 371 us in equal pieces, 230 by samples; grid steps 339 and 740).
 template <class Tr>
 __device__ void sort_ranges(const Scratch& sc, const Window<Tr>& w, uint32_t* smem, uint32_t job0,
                             bool upd) {
   const uint32_t lane = threadIdx.x & 31, g = gridDim.x;
   // no mutation lies before it (0 when it was not recorded)
   const uint32_t inv = ld_settled(&w.cnt->inv_first_mut), first = inv ? min(~inv, w.n) : 0u;
-  const uint32_t H = huge_groups(sc, w.cnt);
+  const uint32_t H = huge_groups(sc, w.cnt), limit = steps_limit(w);
   uint32_t job = job0 % g, used = 0;  // jobs and seg entries of the groups before
   bool crowded = H > 32;
   for (uint32_t h0 = 0; h0 < H; h0 += 32) {
@@ -1533,10 +1559,11 @@ __device__ void sort_ranges(const Scratch& sc, const Window<Tr>& w, uint32_t* sm
     if (h0 + lane < H) {
       gs = ld_cg_u32(&sc.hlist[h0 + lane]) & sc.gmask;
       cs = min(g_count(ld_relaxed_u64(&sc.gtab[gs])), w.n);
-      if (cs > kHugeSteps || cs <= kHugeMin) cs = 0;
+      if (cs > limit || cs <= kHugeMin) cs = 0;
     }
     crowded |= __reduce_add_sync(0xFFFFFFFFu, cs) / kRangeMembers > g;
     const uint32_t share = crowded ? 2 * kRangeMembers : kRangeMembers;
+    const uint32_t knots = crowded ? 2 * kSampleStep : kSampleStep;
     for (uint32_t q = 0; q < 32; ++q) {
       const uint32_t c = __shfl_sync(0xFFFFFFFFu, cs, q);
       const uint32_t gslot = __shfl_sync(0xFFFFFFFFu, gs, q);
@@ -1545,10 +1572,10 @@ __device__ void sort_ranges(const Scratch& sc, const Window<Tr>& w, uint32_t* sm
       if (used > sc.max_window) return;  // cannot happen: members are distinct ops
       const uint32_t off = sc.max_window - used;
       const uint32_t ranges = (c + share - 1) / share;
+      const uint32_t step = crowded || c > kSampleMin ? knots : 0;
       for (uint32_t r = (blockIdx.x + g - job) % g; r < ranges; r += g) {
         if (r == 0 && threadIdx.x == 0) sc.goff[gslot] = off;
-        sort_range<Tr>(sc, w, gslot, c, off, first, r, ranges, crowded || c > kSampleMin, upd,
-                       smem);
+        sort_range<Tr>(sc, w, gslot, c, off, first, r, ranges, step, upd, smem);
       }
       job = (job + ranges) % g;
     }
@@ -1596,7 +1623,7 @@ __device__ void phase_sort_big(const Scratch& sc, const Window<Tr>& w, uint32_t*
 }
 
 // ------------------------------------------------------- huge groups (D')
-// A group of more than kHugeSteps members (one key takes much of a window) is
+// A group of more than steps_limit members (one key takes much of a window) is
 // ordered by the whole grid in four steps separated by grid barriers, so no block reads
 // back global data that it wrote itself in the same step:
 //   hist     every warp takes storage units (inline part / 32-member chunks)
@@ -1652,10 +1679,11 @@ template <class Tr>
 __device__ void huge_hist(const Scratch& sc, const Window<Tr>& w, uint32_t gwarp,
                           uint32_t ngwarps) {
   const uint32_t H = huge_groups(sc, w.cnt), width = huge_width(w.n), lane = lane_id();
+  const uint32_t limit = steps_limit(w);
   for (uint32_t h = 0; h < H; ++h) {
     uint32_t gslot;
     const uint32_t c = huge_size(sc, w, h, &gslot);
-    if (c <= kHugeSteps) continue;  // sort_ranges ordered it
+    if (c <= limit) continue;  // sort_ranges ordered it
     const uint32_t units = 1 + (c - kInline + kChunk - 1) / kChunk;
     uint32_t* bins = sc.hbins + (size_t)h * kHugeBins;
     for (uint32_t k = gwarp; k < units; k += ngwarps) {
@@ -1675,14 +1703,14 @@ template <class Tr>
 __device__ void huge_scan(const Scratch& sc, const Window<Tr>& w, uint32_t* smem) {
   __shared__ uint32_t s_off, s_base, s_last, s_tmp[32];
   const uint32_t tid = threadIdx.x, nt = blockDim.x;
-  const uint32_t H = huge_groups(sc, w.cnt);
+  const uint32_t H = huge_groups(sc, w.cnt), limit = steps_limit(w);
   const uint32_t per = (kHugeBins + nt - 1) / nt, b0 = tid * per;
   for (uint32_t h = blockIdx.x; h < H; h += gridDim.x) {
     if (tid == 0) s_last = 0;
     __syncthreads();
     uint32_t gslot;
     const uint32_t c = huge_size(sc, w, h, &gslot);
-    if (c <= kHugeSteps) continue;  // block-uniform
+    if (c <= limit) continue;  // block-uniform
     uint32_t* bins = sc.hbins + (size_t)h * kHugeBins;
     uint32_t* hrun = sc.hrun + (size_t)h * kHugeBins;
     uint32_t local = 0;
@@ -1753,11 +1781,12 @@ template <class Tr>
 __device__ void huge_scatter(const Scratch& sc, const Window<Tr>& w, uint32_t gwarp,
                              uint32_t ngwarps) {
   const uint32_t H = huge_groups(sc, w.cnt), width = huge_width(w.n), lane = lane_id();
+  const uint32_t limit = steps_limit(w);
   const bool upd = ld_settled(&w.cnt->upd_count) != 0;
   for (uint32_t h = 0; h < H; ++h) {
     uint32_t gslot;
     const uint32_t c = huge_size(sc, w, h, &gslot);
-    if (c <= kHugeSteps) continue;  // sort_ranges ordered it
+    if (c <= limit) continue;  // sort_ranges ordered it
     const uint32_t units = 1 + (c - kInline + kChunk - 1) / kChunk;
     uint32_t* bins = sc.hbins + (size_t)h * kHugeBins;
     const uint32_t* hrun = sc.hrun + (size_t)h * kHugeBins;

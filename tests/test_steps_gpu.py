@@ -1,6 +1,6 @@
 """Groups of more than 2^17 mutations, which the whole grid orders in steps with
 barriers between them: two in one window, one whose ops are updates for whole
-runs, through the per-phase, the persistent (both probe orders) and the
+runs, and two and three of more than 98,304, which takes three to the steps, through the per-phase, the persistent (both probe orders) and the
 two-stream form.  Every result and the contents equal the oracle's replay."""
 from __future__ import annotations
 
@@ -21,6 +21,15 @@ def _batch(kind):
     rng = np.random.default_rng(79)
     t = rng.choice([0, 1, 2, 3], size=N, p=[0.25, 0.35, 0.2, 0.2]).astype(np.uint8)
     k = W.key_of_rank(6, rng.integers(0, 3000, size=N))
+    if kind in ("two_mid", "three_mid"):
+        k[:], t[:] = W.key_of_rank(6, np.arange(N) % 3000), 0
+        at, last = rng.permutation(N), 98_304 + (kind == "three_mid")
+        for i, c in enumerate((98_305, 100_001, last, 60_000)):
+            m, at = at[:c], at[c:]
+            k[m], t[m] = np.uint64(1 + i), rng.choice([1, 2, 3], size=c, p=[0.4, 0.2, 0.4])
+            r, at = at[:2000], at[2000:]
+            k[r] = np.uint64(1 + i)
+        return t, k, W.splitmix64(8, 0, N)
     if kind == "two":  # one spread over the window, one in a row; a third below the limit
         k[rng.random(N) < 0.75] = np.uint64(1)
         k[300_000:500_000] = np.uint64(2)
@@ -37,7 +46,7 @@ def _batch(kind):
 
 
 @pytest.mark.parametrize("form", ["plain", "fused", "split0", "overlap"])
-@pytest.mark.parametrize("kind", ["two", "updates"])
+@pytest.mark.parametrize("kind", ["two", "updates", "two_mid", "three_mid"])
 def test_groups_over_the_steps_limit(cuda, kind, form):
     import torch
     t, k, v = _batch(kind)
